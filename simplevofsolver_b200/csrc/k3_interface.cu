@@ -22,6 +22,8 @@
 // are kept from the previous plane.
 #include <cuda_pipeline.h>
 
+#include <type_traits>
+
 #include "svof3d_internal.cuh"
 #include "smem_limit.cuh"
 
@@ -187,23 +189,23 @@ __device__ __forceinline__ void load_normal(const float *__restrict__ normal, lo
 // ---------------------------------------------------------------------------
 // k3_geom: cells i in [1, nx], j in [0, ny+1], k in [0, nz+1] (halo cells
 // included, as the restatement computes them).  Block: 32 x 4 cells of one
-// plane, marching over G3Z planes; shared memory holds a ring of vof planes
+// plane, marching over `planes` planes; shared memory holds a ring of vof planes
 // (34 x 6, FP64), G3D planes in flight ahead of the two being read, and two
 // planes of corner normals (33 x 5 x 3, R).  The vof differences are taken
 // in FP64 and then carried in R.
-constexpr int G3X = 32, G3Y = 4, G3Z = 32, G3D = 4, G3S = G3D + 2;
+constexpr int G3X = 32, G3Y = 4, G3D = 4, G3S = G3D + 2;
 
 template <class R>
 __global__ void __launch_bounds__(G3X * G3Y) k3_geom(const double *__restrict__ vof, R *__restrict__ normal,
                                                     R *__restrict__ curv, unsigned *__restrict__ work,
-                                                    unsigned *__restrict__ nwork, Grid3 g) {
+                                                    unsigned *__restrict__ nwork, int planes, Grid3 g) {
   __shared__ double sv[G3S][G3Y + 2][G3X + 2];  // vof planes, plane p in slot (p - k0 + 1) % G3S
   __shared__ R sc[2][3][G3Y + 1][G3X + 1];
   const int nx = g.nx, ny = g.ny, nz = g.nz;
   const int i0 = 1 + blockIdx.x * G3X;
   const int j0 = blockIdx.y * G3Y;
-  const int k0 = blockIdx.z * G3Z;
-  const int kend = min(k0 + G3Z, nz + 2);  // cells k in [k0, kend)
+  const int k0 = blockIdx.z * planes;
+  const int kend = min(k0 + planes, nz + 2);  // cells k in [k0, kend)
   const int tid = threadIdx.x;
   const int tx = tid % G3X, ty = tid / G3X;
   const R eps = R(kDblEpsilon);
@@ -503,13 +505,15 @@ __device__ __forceinline__ double face_flux(double vel, double vlo, double vhi, 
 // plane.  Writes vof_new with its halo images (two layers) and zero x walls,
 // and src_a.  The flux divergence and the update are FP64 in both
 // precisions, so that the update conserves volume to FP64 round-off.
-constexpr int AX = 32, AY = 8, AZ = 32, AWX = AX + 2, AWY = AY + 2, ASLOT = 4;
+constexpr int AX = 32, AY = 8, AWX = AX + 2, AWY = AY + 2, ASLOT = 4;
 constexpr int kVofRing = ASLOT * AWY * AWX, kUxRing = ASLOT * AY * (AX + 1), kUyRing = ASLOT * (AY + 1) * AX;
 constexpr int kUzRing = ASLOT * AY * AX, kSbRing = ASLOT * AY * AX;
 constexpr size_t kAdvectSmem =
     sizeof(double) * (kVofRing + kUxRing + kUyRing + kUzRing + kSbRing + AY * (AX + 1) + (AY + 1) * AX);
 
-template <class R>
+// AZ is a template parameter: as a kernel argument it costs the FP64 kernel a
+// register it does not have (64 of them, 8 bytes spilled, 512^3 2.54 -> 2.84 ms).
+template <class R, int AZ>
 __global__ void __launch_bounds__(AX * AY, 4) k3_vof_advect(const double *__restrict__ vof, double *__restrict__ vof_new,
                                                         const double *__restrict__ ux, const double *__restrict__ uy,
                                                         const double *__restrict__ uz, const R *__restrict__ normal,
@@ -690,13 +694,26 @@ __global__ void __launch_bounds__(AX * AY, 4) k3_vof_advect(const double *__rest
 }
 
 // ---- host-side launchers
+// f(depth) with the power of two nearest below 4/3 of `planes` (8 for 6 .. 11)
+template <class F>
+cudaError_t by_depth(int planes, F f) {
+  if (planes >= 24) return f(std::integral_constant<int, 32>());
+  if (planes >= 12) return f(std::integral_constant<int, 16>());
+  if (planes >= 6) return f(std::integral_constant<int, 8>());
+  if (planes >= 3) return f(std::integral_constant<int, 4>());
+  if (planes >= 2) return f(std::integral_constant<int, 2>());
+  return f(std::integral_constant<int, 1>());
+}
+
 template <class R>
 cudaError_t interface_geom(cudaStream_t st, const double *vof, R *normal, R *curv, unsigned *work,
                            unsigned *nwork, Grid3 g, unsigned long long *unconverged) {
   cudaError_t e = cudaMemsetAsync(nwork, 0, sizeof(unsigned), st);
   if (cudaSuccess != e) return e;
-  dim3 gr((g.nx + G3X - 1) / G3X, (g.ny + 2 + G3Y - 1) / G3Y, (g.nz + 2 + G3Z - 1) / G3Z);
-  k3_geom<R><<<gr, G3X * G3Y, 0, st>>>(vof, normal, curv, work, nwork, g);
+  const long columns = (long)((g.nx + G3X - 1) / G3X) * ((g.ny + 2 + G3Y - 1) / G3Y);
+  const int planes = march_planes_uneven(columns, g.nz + 2, 32, 7);
+  dim3 gr((g.nx + G3X - 1) / G3X, (g.ny + 2 + G3Y - 1) / G3Y, (g.nz + 2 + planes - 1) / planes);
+  k3_geom<R><<<gr, G3X * G3Y, 0, st>>>(vof, normal, curv, work, nwork, planes, g);
   if (cudaSuccess != (e = cudaGetLastError())) return e;
   k3_intercept<R><<<148 * 8, 256, 0, st>>>(vof, normal, work, nwork, g, unconverged);
   return cudaGetLastError();
@@ -714,14 +731,26 @@ template <class R>
 cudaError_t interface_advect(cudaStream_t st, const double *vof, double *vof_new, const double *ux,
                              const double *uy, const double *uz, const R *normal, double *src_a,
                              const double *src_b, const double *dtp, RK rk, int use_b, Grid3 g) {
-  dim3 gr((g.nx + AX - 1) / AX, (g.ny + AY - 1) / AY, (g.nz + AZ - 1) / AZ);
-  k3_vof_advect<R><<<gr, AX * AY, kAdvectSmem, st>>>(vof, vof_new, ux, uy, uz, normal, src_a, src_b, dtp, rk, use_b, g);
+  const int planes = march_planes_uneven((long)((g.nx + AX - 1) / AX) * ((g.ny + AY - 1) / AY), g.nz, 32, 4);
+  by_depth(planes, [&](auto c) {
+    constexpr int AZ = decltype(c)::value;
+    dim3 gr((g.nx + AX - 1) / AX, (g.ny + AY - 1) / AY, (g.nz + AZ - 1) / AZ);
+    k3_vof_advect<R, AZ><<<gr, AX * AY, kAdvectSmem, st>>>(vof, vof_new, ux, uy, uz, normal, src_a, src_b, dtp, rk,
+                                                           use_b, g);
+    return cudaSuccess;
+  });
   return cudaGetLastError();
 }
 
 template <class R>
 cudaError_t interface_prepare_t() {
-  return raise_smem_limit(k3_vof_advect<R>, kAdvectSmem);
+  for (int d = 1; d <= 32; d *= 2) {
+    const cudaError_t e = by_depth(d, [](auto c) {
+      return raise_smem_limit(k3_vof_advect<R, decltype(c)::value>, kAdvectSmem);
+    });
+    if (cudaSuccess != e) return e;
+  }
+  return cudaSuccess;
 }
 
 #define SVOF3_INTERFACE_INST(R)                                                                                \

@@ -270,14 +270,14 @@ __device__ __forceinline__ void rhs4_values(const Predict3Args<R> &a, const Grid
 
 // ---------------------------------------------------------------------------
 // k3_rhs: the right-hand sides and increments of all cells.  A block owns a
-// 32 x 8 tile of (i, j) and marches along z over RZ planes.  The five state
+// 32 x 8 tile of (i, j) and marches along z over `planes` planes.  The five state
 // fields ux, uy, uz, t, p live in a ring of four shared-memory planes (a
 // 34 x 10 window each, the tile with its x and y neighbours): planes k - 1,
 // k, k + 1 are read by the stencil while plane k + 2 arrives by cp.async.
 // Writes src_a and the increment delta = dt (alpha src_a + beta src_b +
 // gamma src_g) in the line layout [field][j - 1 + ny (k - 1)][x position]
 // that the line solver reads.
-constexpr int RX = 32, RY = 8, RZ = 64;
+constexpr int RX = 32, RY = 8;
 constexpr int WX = RX + 2, WY = RY + 2, NSLOT = 4, NFLD = 5, NCEN = 7;
 // the state windows (FP64) and the per-cell inputs ifrcx / ifrcy / ifrcz and
 // src_b of the four fields (R-sized: 83 KB per mixed block instead of 112 KB,
@@ -294,13 +294,13 @@ constexpr size_t kRhsSmem =
 // GRAV: the instantiation with the vof buoyancy extension (grav_vof != 0);
 // the other one is the reference's right-hand side alone
 template <class R, bool GRAV>
-__global__ void __launch_bounds__(RX * RY, 2) k3_rhs(Predict3Args<R> a) {
+__global__ void __launch_bounds__(RX * RY, 2) k3_rhs(Predict3Args<R> a, int planes) {
   extern __shared__ double ring[];  // [NFLD][NSLOT][WY][WX]
   const Grid3 g = a.g;
   const int nx = g.nx, ny = g.ny, nz = g.nz;
   const int tid = threadIdx.x, tx = tid % RX, ty = tid / RX;
-  const int i0 = 1 + blockIdx.x * RX, j0 = 1 + blockIdx.y * RY, k0 = 1 + blockIdx.z * RZ;
-  const int kend = min(k0 + RZ, nz + 1);  // cells k in [k0, kend)
+  const int i0 = 1 + blockIdx.x * RX, j0 = 1 + blockIdx.y * RY, k0 = 1 + blockIdx.z * planes;
+  const int kend = min(k0 + planes, nz + 1);  // cells k in [k0, kend)
   const int i = i0 + tx, j = j0 + ty;
   const bool mine = i <= nx && j <= ny;
   const bool do_ux = i < nx;
@@ -689,9 +689,10 @@ __global__ void __launch_bounds__(256) k3_xsolve(Predict3Args<R> a) {
 template <class R>
 cudaError_t predict_launch(cudaStream_t st, const Predict3Args<R> &a) {
   const Grid3 &g = a.g;
-  dim3 gr((g.nx + RX - 1) / RX, (g.ny + RY - 1) / RY, (g.nz + RZ - 1) / RZ);
-  if (0. != a.grav_vof) k3_rhs<R, true><<<gr, RX * RY, kRhsSmem<R>, st>>>(a);
-  else k3_rhs<R, false><<<gr, RX * RY, kRhsSmem<R>, st>>>(a);
+  const int planes = march_planes_even((long)((g.nx + RX - 1) / RX) * ((g.ny + RY - 1) / RY), g.nz, 64, 2, 3);
+  dim3 gr((g.nx + RX - 1) / RX, (g.ny + RY - 1) / RY, (g.nz + planes - 1) / planes);
+  if (0. != a.grav_vof) k3_rhs<R, true><<<gr, RX * RY, kRhsSmem<R>, st>>>(a, planes);
+  else k3_rhs<R, false><<<gr, RX * RY, kRhsSmem<R>, st>>>(a, planes);
   cudaError_t e = cudaGetLastError();
   if (cudaSuccess != e) return e;
   const long nlines = (long)g.ny * g.nz;

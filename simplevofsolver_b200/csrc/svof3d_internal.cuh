@@ -6,6 +6,8 @@
 
 #include <cuda_runtime.h>
 #include <cstddef>
+#include <algorithm>
+#include <cmath>
 #include <cstdint>
 
 #include "../../include/svof3d_b200.h"
@@ -211,5 +213,41 @@ constexpr int kPredLines = 32;  // lines per predictor block
 constexpr int kPredChunk = 32;  // x positions per chunk
 constexpr int kProjectPlanes = 4;  // z planes per thread of k3_project
 constexpr int kCflPlanes = 8;      // z planes per thread of k3_cfl (blocks of 32 x 8)
+
+// Planes per block of a kernel whose blocks march along z: `columns` blocks
+// tile a plane, `resident` of them fit an SM.  Shallow blocks repeat their
+// prologue (the planes around the first one) more often, deep ones leave the
+// chip idle.  Two rules, by the kernel's kind (both sides measured, us a
+// launch; the fixed depths before: right-hand sides 64, the others 32).
+//
+// Blocks of equal cost (k3_rhs): the depth up to `most` with the least waves
+// x (planes + lead), the blocks of a wave running side by side.  61 x 64 x 32
+// 68.6 -> 11.2 (2 planes; 1: 14.3), 256^3 656 -> 624 (32; 16: 633), 512^3
+// unchanged (64).
+inline int march_planes_even(long columns, int nz, int most, int resident, int lead) {
+  const long slots = 148L * resident;
+  int best = 1;
+  long least = -1;
+  for (int seg = (nz + most - 1) / most; seg <= nz; seg++) {
+    const int d = (nz + seg - 1) / seg;
+    const long cost = ((columns * ((nz + d - 1) / d) + slots - 1) / slots) * (d + lead);
+    if (least < 0 || cost < least) {
+      least = cost;
+      best = d;
+    }
+  }
+  return best;
+}
+
+// Blocks whose cost depends on the interface they hold (k3_geom,
+// k3_vof_advect): work grows as 1 + lead / d, the tail of uneven blocks as
+// d, hence the square root; 1.2 is the ratio of the two.  Vof advection 61 x
+// 64 x 32 98 -> 12.6 (1 plane; 2: 18.1), 128^3 mixed 86 -> 53.7 (4; 8:
+// 56.8), 256^3 449 -> 423 (8; 19: 445), 512^3 unchanged (32);
+// geometry 34.4 -> 9.2, 47.9 -> 27.1, 165 -> 151, unchanged.
+inline int march_planes_uneven(long columns, int nz, int most, int resident) {
+  const double d = std::sqrt(1.2 * (double)columns * nz / (148. * resident));
+  return std::max(1, std::min({most, nz, (int)(d + 0.5)}));
+}
 
 }  // namespace svof3
