@@ -12,10 +12,13 @@
 //   k3_pois_fwd_y  a block owns COLS consecutive i of one plane k
 //   k3_pois_z      a block owns COLS consecutive i of one ky, both signs
 //                  (in place)
-//   k3_pois_x      a block owns 64 or 128 lines (ky, kz), one per thread,
-//                  walked in 16-cell chunks: forward recurrence (values back
-//                  into S, v into scratch), then back substitution in reverse
-//                  chunk order
+//   x line solves  cline_solve.cuh (whole lines in shared memory, the pivots
+//                  from a table made at the solver's creation), or, for more
+//                  lines than those cover in a few rounds, k3_pois_x: a block
+//                  owns 64 or 128 lines (ky, kz), one per thread, walked in
+//                  16-cell chunks: forward recurrence (values back into S, v
+//                  into scratch), then back substitution in reverse chunk
+//                  order
 //   k3_pois_inv_y  a block owns COLS consecutive i of one plane k; writes psi
 //                  with its halo images and Neumann walls
 //
@@ -32,6 +35,7 @@
 
 #include <type_traits>
 
+#include "cline_solve.cuh"
 #include "fft_device.cuh"
 #include "svof3d_internal.cuh"
 #include "smem_limit.cuh"
@@ -602,8 +606,21 @@ cudaError_t line_attrs(K kernel, int smem) {
 }
 }  // namespace
 
+// whole lines in shared memory where the chip takes all of them in at most
+// 12 rounds: beyond that the chip holds too few lines at a time (their
+// latency, not the bytes, is then what counts) and k3_pois_x streams near the
+// copy rate.  us a launch, whole lines against k3_pois_x: 61 x 64 x 32 10 /
+// 28, 128^3 18 / 53, 256^3 (6 rounds) 116 / 153, 512^3 (44) 1300 / 955.
+static bool pois_x_whole_lines(long nlines, int nx) {
+  const int lpb = svof_cline::cline_lpb(nlines, nx, sizeof(double));
+  const size_t bytes = svof_cline::cline_smem(lpb, nx, sizeof(double)) + 1024;
+  if (bytes > 227 * 1024) return false;
+  const long held = 148L * lpb * std::min<long>(32, 227 * 1024 / bytes);
+  return nlines <= 12 * held;
+}
+
 template <class R>
-cudaError_t pois_prepare(int log2ny, int log2nz) {
+cudaError_t pois_prepare(int nx, int log2ny, int log2nz) {
   if (log2ny < kMinL2N || log2ny > kMaxL2N || log2nz < kMinL2N || log2nz > kMaxL2N) return cudaErrorInvalidValue;
   cudaError_t e = by_l2n(log2ny, [&](auto c) {
     constexpr int L2 = decltype(c)::value;
@@ -623,6 +640,8 @@ cudaError_t pois_prepare(int log2ny, int log2nz) {
     return line_attrs(k3_pois_z<L2, R>, Line<R, L2>::SMEM);
   });
   if (cudaSuccess != e) return e;
+  const long nlines = (long)((1 << log2ny) / 2 + 1) << log2nz;
+  if (pois_x_whole_lines(nlines, nx)) return svof_cline::cline_prepare<R>(nlines, nx);
   if (cudaSuccess != (e = line_attrs(k3_pois_x<R, 64>, (int)XShape<R, 64>::SMEM))) return e;
   return line_attrs(k3_pois_x<R, 128>, (int)XShape<R, 128>::SMEM);
 }
@@ -654,14 +673,36 @@ cudaError_t pois_z(cudaStream_t st, R *spec, const R *tw, int log2n, Grid3 g) {
   });
 }
 
-// lines per block of the x solve: 128, or 64 when 128 would leave SMs idle
+cudaError_t pois_x_table(cudaStream_t st, double *tab, const double *pl, const double *pu, const double *evy,
+                         const double *evz, Grid3 g, unsigned long long *nsmall) {
+  using namespace svof_cline;
+  const int nky = g.ny / 2 + 1;
+  const long nlines = (long)nky * g.nz;
+  if (!pois_x_whole_lines(nlines, g.nx)) return cudaSuccess;
+  k_cline_table<<<(unsigned)((nlines + kTabLines - 1) / kTabLines), kTabLines, 0, st>>>(tab, pl, pu, evy, evz, nky,
+                                                                                       nlines, g.nx, nsmall);
+  return cudaGetLastError();
+}
+
+// lines per block of k3_pois_x: 128, or 64 when 128 would leave SMs idle
 inline bool pois_x_narrow(long nlines) { return nlines < 148L * 4 * 128; }
 
 template <class R>
-cudaError_t pois_x(cudaStream_t st, R *spec, R *scratch, const double *pl, const double *pu, const double *evy,
-                   const double *evz, Grid3 g, bool gauge0, unsigned long long *small_pivots) {
+cudaError_t pois_x(cudaStream_t st, R *spec, double *aux, const double *pl, const double *pu, const double *evy,
+                   const double *evz, Grid3 g, bool gauge0, unsigned long long *small_pivots,
+                   const unsigned long long *nsmall) {
+  using namespace svof_cline;
   const long nlines = (long)(g.ny / 2 + 1) * g.nz;
   const int gz = gauge0 ? 1 : 0;
+  if (pois_x_whole_lines(nlines, g.nx)) {
+    return cline_by_lpb(cline_lpb(nlines, g.nx, sizeof(R)), [&](auto c) {
+      constexpr int LPB = decltype(c)::value;
+      k_cline_solve<R, LPB><<<(unsigned)((nlines + LPB - 1) / LPB), 32, cline_smem(LPB, g.nx, sizeof(R)), st>>>(
+          spec, aux, pl, pu, nlines, g.nx, gz, small_pivots, nsmall);
+      return cudaGetLastError();
+    });
+  }
+  R *scratch = reinterpret_cast<R *>(aux);
   if (pois_x_narrow(nlines)) {
     k3_pois_x<R, 64><<<(unsigned)((nlines + 63) / 64), 64, XShape<R, 64>::SMEM, st>>>(spec, scratch, pl, pu, evy,
                                                                                       evz, g, gz, small_pivots);
@@ -730,12 +771,12 @@ cudaError_t pois_resid(cudaStream_t st, const double *b, const double *psi, doub
 }
 
 #define SVOF3_POISSON_INST(R)                                                                                    \
-  template cudaError_t pois_prepare<R>(int, int);                                                                \
+  template cudaError_t pois_prepare<R>(int, int, int);                                                           \
   template cudaError_t pois_fwd_y<R>(cudaStream_t, const double *, const double *, const double *, double *, R *, \
                                      const R *, const double *, double, int, Grid3);                            \
   template cudaError_t pois_z<R>(cudaStream_t, R *, const R *, int, Grid3);                                      \
-  template cudaError_t pois_x<R>(cudaStream_t, R *, R *, const double *, const double *, const double *,        \
-                                 const double *, Grid3, bool, unsigned long long *);                             \
+  template cudaError_t pois_x<R>(cudaStream_t, R *, double *, const double *, const double *, const double *,   \
+                                 const double *, Grid3, bool, unsigned long long *, const unsigned long long *); \
   template cudaError_t pois_inv_y<R>(cudaStream_t, const R *, double *, const R *, int, Grid3, bool);          \
   template cudaError_t pois_fwd_y_array<R>(cudaStream_t, const double *, R *, const R *, int, Grid3);
 SVOF3_POISSON_INST(double)

@@ -116,7 +116,7 @@ struct svof3d_solver {
   double lapy[3] = {0., 0., 0.}, lapz[3] = {0., 0., 0.};
   double lims[4] = {0., 0., 0., 0.};  // explicit diffusive dt limits: m y, m z, t y, t z
   // Poisson
-  DevBuf spec, xscratch, twf_y, twb_y, twf_z, twb_z, pl, pu, evy, evz;
+  DevBuf spec, xaux, twf_y, twb_y, twf_z, twb_z, pl, pu, evy, evz;
   DevBuf twf_y32, twb_y32, twf_z32, twb_z32;  // FP32 twiddles (SVOF3_MIXED_DC)
   // predictor forward-sweep scratch
   DevBuf fw;
@@ -129,7 +129,8 @@ struct svof3d_solver {
   unsigned *d_status = nullptr;
   // health counters, accumulated until svof3d_health resets them: [0] THINC
   // intercepts whose Newton iteration did not converge, [1] Poisson x lines
-  // (other than ky = kz = 0) that met a pivot of magnitude <= DBL_EPSILON
+  // (other than ky = kz = 0) that met a pivot of magnitude <= DBL_EPSILON;
+  // [2] how many lines of one solve do (a property of the grid, set at creation)
   unsigned long long *d_health = nullptr;
   double *h_dt = nullptr;
   int h_dt_slots = 0;
@@ -317,7 +318,7 @@ int launch_potential_dc(svof3d_solver *s, int rk, const Marker &mark) {
   auto m = [&](int kind) { return mark ? mark(kind) : 0; };
   const int cu = s->cur_u;
   double *b = s->fw.as<double>(), *r = b + (size_t)s->nx * s->ny * s->nz;
-  float *sp = s->spec.as<float>(), *xs = s->xscratch.as<float>();
+  float *sp = s->spec.as<float>();
   for (int pass = 0; pass < 2; pass++) {
     if (0 == pass) {
       CK(pois_fwd_y<float>(s->stream, s->ux[cu].p, s->uy[cu].p, s->uz[cu].p, b, sp, s->twf_y32.as<float>(),
@@ -329,7 +330,8 @@ int launch_potential_dc(svof3d_solver *s, int rk, const Marker &mark) {
     if (m(SVOF3_K_POISSON_FWD)) return 1;
     CK(pois_z<float>(s->stream, sp, s->twf_z32.as<float>(), s->log2nz, g));
     if (m(SVOF3_K_POISSON_Z)) return 1;
-    CK(pois_x<float>(s->stream, sp, xs, s->pl.p, s->pu.p, s->evy.p, s->evz.p, g, true, s->d_health + 1));
+    CK(pois_x<float>(s->stream, sp, s->xaux.p, s->pl.p, s->pu.p, s->evy.p, s->evz.p, g, true, s->d_health + 1,
+                     s->d_health + 2));
     if (m(SVOF3_K_POISSON_SOLVE)) return 1;
     CK(pois_z<float>(s->stream, sp, s->twb_z32.as<float>(), s->log2nz, g));
     if (m(SVOF3_K_POISSON_Z)) return 1;
@@ -360,8 +362,8 @@ int launch_potential(svof3d_solver *s, int rk, const Marker &mark = Marker()) {
   if (m(SVOF3_K_POISSON_FWD)) return 1;
   CK(pois_z<double>(s->stream, s->spec.p, s->twf_z.p, s->log2nz, g));
   if (m(SVOF3_K_POISSON_Z)) return 1;
-  CK(pois_x<double>(s->stream, s->spec.p, s->xscratch.p, s->pl.p, s->pu.p, s->evy.p, s->evz.p, g, false,
-                    s->d_health + 1));
+  CK(pois_x<double>(s->stream, s->spec.p, s->xaux.p, s->pl.p, s->pu.p, s->evy.p, s->evz.p, g, false,
+                    s->d_health + 1, s->d_health + 2));
   if (m(SVOF3_K_POISSON_SOLVE)) return 1;
   CK(pois_z<double>(s->stream, s->spec.p, s->twb_z.p, s->log2nz, g));
   if (m(SVOF3_K_POISSON_Z)) return 1;
@@ -583,7 +585,7 @@ int svof3d_destroy(svof3d_solver_t *s) {
     dfree(s->sux[k]); dfree(s->suy[k]); dfree(s->suz[k]); dfree(s->st[k]); dfree(s->svof[k]);
   }
   DevBuf *bufs[] = {&s->p, &s->psi, &s->curv, &s->normal, &s->ifrcx, &s->ifrcy, &s->ifrcz, &s->dxf, &s->dxc,
-                    &s->lap_ux, &s->lap_cc, &s->coef, &s->spec, &s->xscratch, &s->twf_y, &s->twb_y, &s->twf_z,
+                    &s->lap_ux, &s->lap_cc, &s->coef, &s->spec, &s->xaux, &s->twf_y, &s->twb_y, &s->twf_z,
                     &s->twb_z, &s->pl, &s->pu, &s->evy, &s->evz, &s->fw, &s->diag, &s->stat_part,
                     &s->twf_y32, &s->twb_y32, &s->twf_z32, &s->twb_z32};
   for (DevBuf *b : bufs) dfree(*b);
@@ -649,12 +651,12 @@ int svof3d_create(const svof3d_params_t *prm, const double *xf, const double *xc
   if (build_tables(s, xf, xc)) return bail();
   if (dalloc(s->coef, 9 * nx)) return bail();
   const size_t nky = ny / 2 + 1;
-  if (dalloc(s->spec, 2 * nx * nky * nz) || dalloc(s->xscratch, nx * nky * nz) ||
+  if (dalloc(s->spec, 2 * nx * nky * nz) || dalloc(s->xaux, nx * nky * nz) ||
       dalloc(s->fw, 4 * nx * ny * nz, es))
     return bail();
   {
     const cudaError_t pe =
-        s->dc ? pois_prepare<float>(s->log2ny, s->log2nz) : pois_prepare<double>(s->log2ny, s->log2nz);
+        s->dc ? pois_prepare<float>(s->nx, s->log2ny, s->log2nz) : pois_prepare<double>(s->nx, s->log2ny, s->log2nz);
     if (cudaSuccess != pe || cudaSuccess != predict_prepare() || cudaSuccess != interface_prepare())
       return fail("cudaFuncSetAttribute(Poisson): %s", cudaGetErrorString(cudaGetLastError())), bail();
     const size_t coef_smem = sizeof(double) * 6 * nx;
@@ -668,9 +670,13 @@ int svof3d_create(const svof3d_params_t *prm, const double *xf, const double *xc
   if (cudaSuccess != cudaMalloc(&s->d_minbits, sizeof(unsigned long long))) return fail("cudaMalloc"), bail();
   if (cudaSuccess != cudaMalloc(&s->d_status, sizeof(unsigned)) ||
       cudaSuccess != cudaMemset(s->d_status, 0, sizeof(unsigned)) ||
-      cudaSuccess != cudaMalloc(&s->d_health, 2 * sizeof(unsigned long long)) ||
-      cudaSuccess != cudaMemset(s->d_health, 0, 2 * sizeof(unsigned long long)))
+      cudaSuccess != cudaMalloc(&s->d_health, 3 * sizeof(unsigned long long)) ||
+      cudaSuccess != cudaMemset(s->d_health, 0, 3 * sizeof(unsigned long long)))
     return fail("cudaMalloc status"), bail();
+  if (cudaSuccess != cudaDeviceSynchronize() ||
+      cudaSuccess != pois_x_table(s->stream, s->xaux.p, s->pl.p, s->pu.p, s->evy.p, s->evz.p, s->grid(),
+                                  s->d_health + 2))
+    return fail("svof3d_create: Poisson pivots: %s", cudaGetErrorString(cudaGetLastError())), bail();
   {
     const double one = 1.;
     unsigned long long bits;
@@ -1227,7 +1233,7 @@ int adj3_ensure(svof3d_solver *s) {
   if (!bad && a->f32) bad = dalloc(a->zx, nf) || dalloc(a->zy, nc) || dalloc(a->zz, nc);
   if (!bad && s->mixed)
     bad = dalloc(a->nrm64, 4 * nx * (ny + 2) * (nz + 2)) || dalloc(a->curv64, ncc) ||
-          (s->dc && cudaSuccess != pois_prepare<double>(s->log2ny, s->log2nz));
+          (s->dc && cudaSuccess != pois_prepare<double>(s->nx, s->log2ny, s->log2nz));
   a->xs_smem = adj_xsolve_smem((int)nx);
   // (FP32 intermediates take the floor too: the exact transposes carry values
   // up to ~1e9 at corners of round-off gradients, beyond FP32's resolution)
@@ -1301,7 +1307,7 @@ int adj3_potential(svof3d_solver *s, int rk, double dt) {
   CK_LAUNCH();
   CK(pois_fwd_y_array<double>(s->stream, a->b.p, s->spec.p, s->twf_y.p, s->log2ny, g));
   CK(pois_z<double>(s->stream, s->spec.p, s->twf_z.p, s->log2nz, g));
-  CK(pois_x<double>(s->stream, s->spec.p, s->xscratch.p, s->pl.p, s->pu.p, s->evy.p, s->evz.p, g, false));
+  CK(pois_x<double>(s->stream, s->spec.p, s->xaux.p, s->pl.p, s->pu.p, s->evy.p, s->evz.p, g));
   CK(pois_z<double>(s->stream, s->spec.p, s->twb_z.p, s->log2nz, g));
   CK(pois_inv_y<double>(s->stream, s->spec.p, a->psis.p, s->twb_y.p, s->log2ny, g, false));
   const double pre_p = 1. / (gam * dt) / (1. * s->ny * s->nz);

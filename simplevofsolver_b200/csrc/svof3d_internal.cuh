@@ -157,19 +157,26 @@ __global__ void k3_tdm_coef(const double *__restrict__ lap_ux, const double *__r
 // solve is FP64.  The transforms are compiled for each length 2^1 .. 2^11
 // (log2n outside that range is an invalid value).
 template <class R>
-cudaError_t pois_prepare(int log2ny, int log2nz);
+cudaError_t pois_prepare(int nx, int log2ny, int log2nz);
 // (b: scratch of nx ny nz doubles for the right-hand side)
 template <class R>
 cudaError_t pois_fwd_y(cudaStream_t st, const double *ux, const double *uy, const double *uz, double *b, R *spec,
                        const R *tw, const double *dtp, double gam, int log2n, Grid3 g);
 template <class R>
 cudaError_t pois_z(cudaStream_t st, R *spec, const R *tw, int log2n, Grid3 g);
+// the x line solves' pivots into aux (nx per line, cline_solve.cuh) where
+// pois_x takes whole lines, and the number of lines other than ky = kz = 0
+// that meet one of magnitude at most DBL_EPSILON (+= *nsmall)
+cudaError_t pois_x_table(cudaStream_t st, double *aux, const double *pl, const double *pu, const double *evy,
+                         const double *evz, Grid3 g, unsigned long long *nsmall);
+// (aux: pois_x_table's, or scratch, nx doubles per line; gauge0: the ky = kz =
+// 0 line takes the gauge psi_hat(last) = 0, for FP32 storage; small_pivots,
+// when given: += the lines other than ky = kz = 0 that met a pivot of
+// magnitude at most DBL_EPSILON)
 template <class R>
-// (gauge0: the ky = kz = 0 line takes the gauge psi_hat(last) = 0, for FP32 storage;
-// small_pivots, when given: += the lines other than ky = kz = 0 that met a
-// pivot of magnitude at most DBL_EPSILON)
-cudaError_t pois_x(cudaStream_t st, R *spec, R *scratch, const double *pl, const double *pu, const double *evy,
-                   const double *evz, Grid3 g, bool gauge0 = false, unsigned long long *small_pivots = nullptr);
+cudaError_t pois_x(cudaStream_t st, R *spec, double *aux, const double *pl, const double *pu, const double *evy,
+                   const double *evz, Grid3 g, bool gauge0 = false, unsigned long long *small_pivots = nullptr,
+                   const unsigned long long *nsmall = nullptr);
 // acc: psi += the result (the correction pass), the walls' halo images kept
 template <class R>
 cudaError_t pois_inv_y(cudaStream_t st, const R *spec, double *psi, const R *tw, int log2n, Grid3 g,
