@@ -65,9 +65,7 @@ int adj_ensure(svof_solver *s) {
   if (!bad && cudaSuccess != raise_smem_limit(k_adj_xsolve, a->xs_smem)) bad = true;
   // the forward transforms on an array right-hand side share the forward's shapes
   if (!bad && s->uniform && cudaSuccess != dct_prepare(s->log2fft)) bad = true;
-  if (!bad && !s->uniform &&
-      cudaSuccess != raise_smem_limit(k_dft_fwd_rhs, sizeof(double) * 2 * (size_t)ny * s->dft_cols))
-    bad = true;
+  if (!bad && !s->uniform && cudaSuccess != dft_prepare(s->log2fft, nx)) bad = true;
   if (bad) {
     std::string e = g_err;
     DevBuf *bufs[] = {&a->ux, &a->uy, &a->p, &a->vof[0], &a->vof[1], &a->pend_v[0], &a->pend_v[1],
@@ -124,17 +122,14 @@ int adj_potential(svof_solver *s, int rk, double dt) {
     CK_LAUNCH();
     pre_p = 1. / (gam * dt) / (2. * s->nx);
   } else {
-    const int cols = s->dft_cols;
-    const int blocks = (s->nx + cols - 1) / cols;
-    const size_t smem = sizeof(double) * 2 * s->ny * cols;
-    const int nky = s->ny / 2 + 1;
-    k_dft_fwd_rhs<<<blocks, 256, smem, s->stream>>>(a->psib.p, s->spec.p, s->twf.p, s->log2fft, cols, g);
+    const int L = s->log2fft, nky = s->ny / 2 + 1, lpb = dft_xsolve_lines(nky, s->nx);
+    const dim3 cols_grid((s->nx + dft_cols(L) - 1) / dft_cols(L));
+    dft_fwd_rhs_kernel(L)<<<cols_grid, dft_threads(L), dft_smem(L), s->stream>>>(a->psib.p, s->spec.p, s->twf.p, g);
     CK_LAUNCH();
-    const int xkt = s->xsolve_kt;
-    k_dft_xsolve<<<(nky + xkt - 1) / xkt, 128, sizeof(double) * 4 * xkt * s->nx, s->stream>>>(
-        s->spec.p, s->vt.p, s->rvt.p, s->pl.p, s->pu.p, s->evals.p, s->nx, nky, xkt);
+    dft_xsolve_kernel(nky, s->nx)<<<(nky + lpb - 1) / lpb, 32, dft_xsolve_smem(nky, s->nx), s->stream>>>(
+        s->spec.p, s->rvt.p, s->pl.p, s->pu.p, nky, s->nx, 0, nullptr, nullptr);
     CK_LAUNCH();
-    k_dft_inv<<<blocks, 256, smem, s->stream>>>(s->spec.p, a->psis.p, s->twb.p, s->log2fft, cols, g);
+    dft_inv_kernel(L)<<<cols_grid, dft_threads(L), dft_smem(L), s->stream>>>(s->spec.p, a->psis.p, s->twb.p, g);
     CK_LAUNCH();
     pre_p = 1. / (gam * dt) / (1. * s->ny);
   }

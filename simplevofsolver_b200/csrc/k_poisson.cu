@@ -7,21 +7,23 @@
 //   k_dct_inv     FFTW_REDFT01 along x, psi row with halo and Neumann walls
 // Stretched x grid (src/fluid/compute_potential/dft.c:406-468):
 //   k_dft_fwd     right-hand side of a tile of columns, r2c along y
-//   k_dft_xsolve  complex Neumann tri-diagonal system along x for every y
-//                 wavenumber (src/tdm.c:17-50, component-wise)
+//   k_cline_solve (cline_solve.cuh) complex Neumann tri-diagonal system along
+//                 x for every y wavenumber (src/tdm.c:17-50, component-wise)
 //   k_dft_inv     c2r along y, psi columns with halo and walls
 //
 // The reference transposes between x- and y-pencils around every transform;
 // on one device the spectral array is instead laid out so that each line
 // solve reads it coalesced: DCT path [j][kx] (threads over kx walk j), DFT
-// path [i][ky] (threads over ky walk i).  No transpose pass exists.
+// path [ky][i] (contiguous lines).  No transpose pass exists.
 //
 // The transforms are the radix-2 decimation-in-time FFT of the oracle
 // (oracle/svof_fft.c) with the same butterflies and the same twiddle tables,
 // so with FMA contraction disabled they agree with it bit for bit.  Lengths
-// must be powers of two (the DCT path's row transforms: 4 .. 4096 points).
+// must be powers of two (the DCT path's row transforms: 4 .. 4096 points, the
+// DFT path's column transforms: 4 .. 8192).
 #include <type_traits>
 
+#include "cline_solve.cuh"
 #include "fft_device.cuh"
 #include "smem_limit.cuh"
 #include "svof_internal.cuh"
@@ -29,7 +31,6 @@
 namespace svof {
 
 using svof_fft_dev::bitrev;
-using svof_fft_dev::fft_stages;
 
 // assign_input, dct.c:285-315 / dft.c:315-345
 __device__ __forceinline__ double poisson_rhs(const double *__restrict__ ux, const double *__restrict__ uy,
@@ -382,206 +383,180 @@ cudaError_t dct_prepare(int log2n) {
 }
 
 // ---------------------------------------------------------------- DFT path
-// columns i0 .. i0+cols-1 of the right-hand side, r2c along y into spec; the
-// block's dynamic shared memory holds cols * 2 ny doubles
-template <class Rhs>
+// The spectrum is S[ky][i], complex, i fastest: the transforms read and write
+// runs of consecutive i, the x solves (cline_solve.cuh) contiguous lines.  A
+// block owns DftShape<L2N>::COLS consecutive columns i (N = ny = 2^L2N points
+// each) and runs their transforms as the register-blocked passes of
+// fft_device.cuh; the first pass evaluates the right-hand side (or reads the
+// spectrum), the last one writes the results.  COLS: 4 (a 32-byte sector of a
+// row) up to 1024 points, so that a 128-wide grid still makes 32 blocks and
+// three blocks of a 1024-point one fit an SM; 2 and 1 columns above, for the
+// same reason.  us a launch, forward and inverse, against tiles of up to 16
+// columns with one stage per barrier: 128 x 256 10.5 / 7.3 against 33 / 26,
+// 1501 x 2048 99 / 60 against 169 / 159 (x solves 9.8 against 15.5, 82 against
+// 313).
+template <int L2N>
+struct DftShape {
+  static constexpr int N = 1 << L2N;
+  static constexpr int COLS = L2N <= 10 ? 4 : (L2N == 11 ? 2 : 1);
+  static constexpr int PAIRS = COLS * (N >> (L2N < 3 ? L2N : 3));
+  static constexpr int THREADS = PAIRS < 32 ? 32 : (PAIRS > 256 ? 256 : (PAIRS + 31) / 32 * 32);
+  static constexpr int LD = svof_fft_dev::fft_ld(L2N);
+  static constexpr size_t SMEM = sizeof(double) * COLS * 2 * (size_t)LD;
+};
+
+// columns i0 .. i0 + COLS - 1 of the right-hand side, r2c along y into spec
+template <int L2N, class Rhs>
 __device__ __forceinline__ void dft_fwd_cols(const Rhs &rhs, double *__restrict__ spec, const double *__restrict__ tw,
-                                             int log2n, int cols, int nx, int n, int i0) {
-  extern __shared__ double z[];
-  const int nky = n / 2 + 1;
-  const int nc = min(cols, nx - i0 + 1);
-  for (int w = threadIdx.x; w < cols * n; w += blockDim.x) {
-    const int q = w / cols, col = w % cols;
-    const int m = bitrev(q, log2n);
-    double v = 0.;
-    if (col < nc) v = rhs(i0 + col, m + 1);
-    z[2 * (col * n + q)] = v;
-    z[2 * (col * n + q) + 1] = 0.;
-  }
-  __syncthreads();
-  fft_stages(z, log2n, cols, tw);
-  for (int w = threadIdx.x; w < nc * nky; w += blockDim.x) {
-    const int col = w / nky, k = w % nky;
-    const size_t o = 2 * ((size_t)(i0 - 1 + col) * nky + k);
-    spec[o] = z[2 * (col * n + k)];
-    spec[o + 1] = z[2 * (col * n + k) + 1];
-  }
+                                             int nx) {
+  using S = DftShape<L2N>;
+  constexpr int N = S::N, COLS = S::COLS, LD = S::LD;
+  extern __shared__ double dsm[];
+  double *re = dsm, *im = re + COLS * LD;
+  const int i0 = 1 + blockIdx.x * COLS;
+  const int nc = min(COLS, nx - i0 + 1);
+  double2 *out = reinterpret_cast<double2 *>(spec) + (i0 - 1);
+  auto first = [&](int c, int base, auto gc, auto hc, double *xr, double *xi) {
+    constexpr int G = decltype(gc)::value, H = decltype(hc)::value;
+#pragma unroll
+    for (int q = 0; q < G; q++) {
+      xr[q] = (c < nc) ? rhs(i0 + c, bitrev(base + q * H, L2N) + 1) : 0.;
+      xi[q] = 0.;
+    }
+  };
+  auto last = [&](int c, int base, auto gc, auto hc, const double *xr, const double *xi) {
+    constexpr int G = decltype(gc)::value, H = decltype(hc)::value;
+    if (c >= nc) return;
+#pragma unroll
+    for (int q = 0; q < G; q++) {
+      const int k = base + q * H;
+      if (k <= N / 2) out[(size_t)k * nx + c] = make_double2(xr[q], xi[q]);
+    }
+  };
+  svof_fft_dev::fft_lines<double, L2N, COLS, 1, S::THREADS>(re, im, tw, first, last);
 }
 
-// a block owns `cols` consecutive columns i0 .. i0+cols-1 and all ny rows;
-// dynamic shared memory cols * 2 ny doubles
-__global__ void k_dft_fwd(const double *__restrict__ ux, const double *__restrict__ uy,
-                          double *__restrict__ spec, const double *__restrict__ tw,
-                          const double *__restrict__ dtp, double gam, int log2n, int cols, Grid2 g) {
+template <int L2N>
+__global__ void __launch_bounds__(DftShape<L2N>::THREADS)
+    k_dft_fwd(const double *__restrict__ ux, const double *__restrict__ uy, double *__restrict__ spec,
+              const double *__restrict__ tw, const double *__restrict__ dtp, double gam, Grid2 g) {
   pdl_enter();
-  const int n = g.ny;
   const double dt = *dtp;
-  const double prefactor = 1. / (gam * dt) / (1. * n);
-  dft_fwd_cols(DivRhs{ux, uy, g, prefactor}, spec, tw, log2n, cols, g.nx, n, 1 + blockIdx.x * cols);
+  const double prefactor = 1. / (gam * dt) / (1. * (1 << L2N));
+  dft_fwd_cols<L2N>(DivRhs{ux, uy, g, prefactor}, spec, tw, g.nx);
 }
 
-__global__ void k_dft_fwd_rhs(const double *__restrict__ r, double *__restrict__ spec, const double *__restrict__ tw,
-                              int log2n, int cols, Grid2 g) {
-  dft_fwd_cols(ArrayRhs{r, g.dxf, g.nx}, spec, tw, log2n, cols, g.nx, g.ny, 1 + blockIdx.x * cols);
+template <int L2N>
+__global__ void __launch_bounds__(DftShape<L2N>::THREADS)
+    k_dft_fwd_rhs(const double *__restrict__ r, double *__restrict__ spec, const double *__restrict__ tw, Grid2 g) {
+  dft_fwd_cols<L2N>(ArrayRhs{r, g.dxf, g.nx}, spec, tw, g.nx);
 }
 
-// complex Neumann Thomas along x per ky (dft.c:364-395); spec layout [i][ky],
-// vt[i][ky] and rvt[i][ky] hold the reference's v and val for each ky.  A
-// block owns kt consecutive ky lines: all threads stage them and their tables
-// in shared memory, one thread per line runs the recurrences there.
-__global__ void k_dft_xsolve(double *__restrict__ spec, const double *__restrict__ vt,
-                             const double *__restrict__ rvt, const double *__restrict__ pl,
-                             const double *__restrict__ pu, const double *__restrict__ evals, int nx,
-                             int nky, int kt) {
+// c2r along y of COLS columns, extract_output and the psi boundaries
+template <int L2N>
+__global__ void __launch_bounds__(DftShape<L2N>::THREADS)
+    k_dft_inv(const double *__restrict__ spec, double *__restrict__ psi, const double *__restrict__ tw, Grid2 g) {
   pdl_enter();
-  extern __shared__ double sm[];
-  double *sre = sm;                        // [nx][kt]
-  double *sim = sm + (size_t)nx * kt;      // [nx][kt]
-  double *sv = sm + 2 * (size_t)nx * kt;   // [nx][kt]
-  double *sr = sm + 3 * (size_t)nx * kt;   // [nx][kt]
-  const int k0 = blockIdx.x * kt;
-  const int nk = min(kt, nky - k0);
-  const int n = nx;
-  for (int w = threadIdx.x; w < n * kt; w += blockDim.x) {
-    const int i = w / kt, t = w - i * kt;
-    const size_t g = (size_t)i * nky + k0 + t;
-    const bool ok = t < nk;
-    sre[w] = ok ? spec[2 * g] : 0.;
-    sim[w] = ok ? spec[2 * g + 1] : 0.;
-    sv[w] = ok ? vt[g] : 0.;
-    sr[w] = ok ? rvt[g] : 0.;
-  }
-  __syncthreads();
-  const int t = threadIdx.x;
-  if (t < nk) {
-    const double ev = evals[k0 + t];
-#define QR(ii) sre[(size_t)(ii) * kt + t]
-#define QI(ii) sim[(size_t)(ii) * kt + t]
-#define V(ii) sv[(size_t)(ii) * kt + t]
-#define RV(ii) sr[(size_t)(ii) * kt + t]
-    // tdm_c with the Neumann boundary rows
-    double c0 = -pl[0] - pu[0] + ev;
-    c0 += pl[0];
-    double pr = QR(0) / c0, pi = QI(0) / c0;
-    QR(0) = pr;
-    QI(0) = pi;
-#pragma unroll 4
-    for (int i = 1; i < n - 1; i++) {
-      const double l = pl[i];
-      const double val = RV(i);  // 1 / (c_i - l_i v_{i-1})
-      pr = val * (QR(i) - l * pr);
-      pi = val * (QI(i) - l * pi);
-      QR(i) = pr;
-      QI(i) = pi;
-    }
-    {
-      const double l = pl[n - 1];
-      double c = -l - pu[n - 1] + ev;
-      c += pu[n - 1];
-      const double val = c - l * V(n - 2);
-      if (fabs(val) > kDblEpsilon) {
-        QR(n - 1) = 1. / val * (QR(n - 1) - l * pr);
-        QI(n - 1) = 1. / val * (QI(n - 1) - l * pi);
-      } else {
-        QR(n - 1) = 0.;
-        QI(n - 1) = 0.;
-      }
-    }
-    double nr = QR(n - 1), ni = QI(n - 1);
-#pragma unroll 4
-    for (int i = n - 2; i >= 0; i--) {
-      const double v = V(i);
-      nr = QR(i) - v * nr;
-      ni = QI(i) - v * ni;
-      QR(i) = nr;
-      QI(i) = ni;
-    }
-#undef QR
-#undef QI
-#undef V
-#undef RV
-  }
-  __syncthreads();
-  for (int w = threadIdx.x; w < n * kt; w += blockDim.x) {
-    const int i = w / kt, tt = w - i * kt;
-    if (tt < nk) {
-      const size_t g = (size_t)i * nky + k0 + tt;
-      spec[2 * g] = sre[w];
-      spec[2 * g + 1] = sim[w];
-    }
-  }
-}
-
-// c2r along y for a tile of columns, extract_output and the psi boundaries
-__global__ void k_dft_inv(const double *__restrict__ spec, double *__restrict__ psi,
-                          const double *__restrict__ tw, int log2n, int cols, Grid2 g) {
-  pdl_enter();
-  extern __shared__ double z[];
-  const int n = g.ny, nx = g.nx, ny = g.ny;
-  const int nky = n / 2 + 1;
-  const int i0 = 1 + blockIdx.x * cols;
-  const int nc = min(cols, nx - i0 + 1);
-  const bool has_left = (1 == i0), has_right = (i0 + nc - 1 == nx);
-  // old wall values feeding the halo rows (read before any write)
-  double wl1 = 0., wln = 0., wr1 = 0., wrn = 0.;
-  if (0 == threadIdx.x) {
-    if (has_left) {
-      wl1 = psi[ix_cc(nx, 0, 1)];
-      wln = psi[ix_cc(nx, 0, ny)];
-    }
-    if (has_right) {
-      wr1 = psi[ix_cc(nx, nx + 1, 1)];
-      wrn = psi[ix_cc(nx, nx + 1, ny)];
-    }
-  }
+  using S = DftShape<L2N>;
+  constexpr int N = S::N, COLS = S::COLS, LD = S::LD;
+  extern __shared__ double dsm[];
+  double *re = dsm, *im = re + COLS * LD;
+  const int nx = g.nx;
+  const int i0 = 1 + blockIdx.x * COLS;
+  const int nc = min(COLS, nx - i0 + 1);
+  const double2 *in = reinterpret_cast<const double2 *>(spec) + (i0 - 1);
   // Hermitian extension as FFTW's c2r reads it: Im of X_0 and X_{n/2} ignored
-  for (int w = threadIdx.x; w < cols * n; w += blockDim.x) {
-    const int q = w / cols, col = w % cols;
-    const int m = bitrev(q, log2n);
-    double re = 0., im = 0.;
-    if (col < nc) {
-      const size_t base = 2 * ((size_t)(i0 - 1 + col) * nky);
-      if (0 == m) {
-        re = spec[base];
-      } else if (2 * m < n) {
-        re = spec[base + 2 * m];
-        im = spec[base + 2 * m + 1];
-      } else if (2 * m == n) {
-        re = spec[base + 2 * m];
-      } else {
-        re = spec[base + 2 * (n - m)];
-        im = -spec[base + 2 * (n - m) + 1];
-      }
+  auto first = [&](int c, int base, auto gc, auto hc, double *xr, double *xi) {
+    constexpr int G = decltype(gc)::value, H = decltype(hc)::value;
+#pragma unroll
+    for (int q = 0; q < G; q++) {
+      const int m = bitrev(base + q * H, L2N);
+      double2 v = make_double2(0., 0.);
+      if (c < nc) v = in[(size_t)(2 * m <= N ? m : N - m) * nx + c];
+      xr[q] = v.x;
+      xi[q] = (0 == m || 2 * m == N) ? 0. : (2 * m < N ? v.y : -v.y);
     }
-    z[2 * (col * n + q)] = re;
-    z[2 * (col * n + q) + 1] = im;
-  }
+  };
+  auto last = [&](int c, int base, auto gc, auto hc, const double *xr, const double *) {
+    constexpr int G = decltype(gc)::value, H = decltype(hc)::value;
+    if (c >= nc) return;
+#pragma unroll
+    for (int q = 0; q < G; q++) {
+      const int j = base + q * H + 1;
+      psi[ix_cc(nx, i0 + c, j)] = xr[q];
+      if (N == j) psi[ix_cc(nx, i0 + c, 0)] = xr[q];
+      if (1 == j) psi[ix_cc(nx, i0 + c, N + 1)] = xr[q];
+    }
+  };
+  svof_fft_dev::fft_lines<double, L2N, COLS, 1, S::THREADS>(re, im, tw, first, last);
+  // Neumann walls, psi.c:7-20 (the blocks at either end of x): the wall cell
+  // takes its neighbour's new value, read back after the barrier, and hands
+  // its old value to the halo row's wall cell
+  const bool has_left = (1 == i0), has_right = (i0 + nc - 1 == nx);
+  if (!has_left && !has_right) return;
   __syncthreads();
-  fft_stages(z, log2n, cols, tw);
-  for (int w = threadIdx.x; w < nc * n; w += blockDim.x) {
-    const int r = w / nc, col = w % nc;
-    const int i = i0 + col, j = r + 1;
-    const double y = z[2 * (col * n + r)];
-    psi[ix_cc(nx, i, j)] = y;
-    if (ny == j) psi[ix_cc(nx, i, 0)] = y;
-    if (1 == j) psi[ix_cc(nx, i, ny + 1)] = y;
+  for (int w = threadIdx.x; w < 2 * N; w += S::THREADS) {
+    const int side = w >> L2N, j = 1 + (w & (N - 1));
+    if (side ? !has_right : !has_left) continue;
+    const int iw = side ? nx + 1 : 0;
+    const double old = psi[ix_cc(nx, iw, j)];
+    psi[ix_cc(nx, iw, j)] = psi[ix_cc(nx, side ? nx : 1, j)];
+    if (N == j) psi[ix_cc(nx, iw, 0)] = old;
+    if (1 == j) psi[ix_cc(nx, iw, N + 1)] = old;
   }
-  __syncthreads();
-  if (0 == threadIdx.x) {
-    if (has_left) {
-      psi[ix_cc(nx, 0, 0)] = wln;
-      psi[ix_cc(nx, 0, ny + 1)] = wl1;
-    }
-    if (has_right) {
-      psi[ix_cc(nx, nx + 1, 0)] = wrn;
-      psi[ix_cc(nx, nx + 1, ny + 1)] = wr1;
-    }
-  }
-  // Neumann walls, psi.c:7-20
-  for (int j = 1 + threadIdx.x; j <= ny; j += blockDim.x) {
-    if (has_left) psi[ix_cc(nx, 0, j)] = z[2 * (0 * n + (j - 1))];
-    if (has_right) psi[ix_cc(nx, nx + 1, j)] = z[2 * ((nc - 1) * n + (j - 1))];
-  }
+}
+
+// ---- launch plans of the DFT column transforms, by length
+namespace {
+template <class F>
+auto dft_by_log2n(int l2n, F f) {
+  if (13 == l2n) return f(std::integral_constant<int, 13>());
+  return by_log2n(l2n, f);
+}
+}  // namespace
+
+bool dft_length_ok(int log2n) { return log2n >= kDctMinL2N && log2n <= kDftMaxL2N; }
+int dft_cols(int log2n) {
+  return dft_by_log2n(log2n, [](auto c) { return DftShape<decltype(c)::value>::COLS; });
+}
+int dft_threads(int log2n) {
+  return dft_by_log2n(log2n, [](auto c) { return DftShape<decltype(c)::value>::THREADS; });
+}
+size_t dft_smem(int log2n) {
+  return dft_by_log2n(log2n, [](auto c) { return DftShape<decltype(c)::value>::SMEM; });
+}
+DftFwdKernel dft_fwd_kernel(int log2n) {
+  return dft_by_log2n(log2n, [](auto c) { return (DftFwdKernel)&k_dft_fwd<decltype(c)::value>; });
+}
+DftFwdRhsKernel dft_fwd_rhs_kernel(int log2n) {
+  return dft_by_log2n(log2n, [](auto c) { return (DftFwdRhsKernel)&k_dft_fwd_rhs<decltype(c)::value>; });
+}
+DftInvKernel dft_inv_kernel(int log2n) {
+  return dft_by_log2n(log2n, [](auto c) { return (DftInvKernel)&k_dft_inv<decltype(c)::value>; });
+}
+DftXSolveKernel dft_xsolve_kernel(long nlines, int nx) {
+  return svof_cline::cline_by_lpb(svof_cline::cline_lpb(nlines, nx, sizeof(double)), [](auto c) {
+    return (DftXSolveKernel)&svof_cline::k_cline_solve<double, decltype(c)::value>;
+  });
+}
+int dft_xsolve_lines(long nlines, int nx) { return svof_cline::cline_lpb(nlines, nx, sizeof(double)); }
+size_t dft_xsolve_smem(long nlines, int nx) {
+  return svof_cline::cline_smem(dft_xsolve_lines(nlines, nx), nx, sizeof(double));
+}
+cudaError_t dft_prepare(int log2n, int nx) {
+  if (!dft_length_ok(log2n)) return cudaErrorInvalidValue;
+  cudaError_t e = raise_smem_limit(dft_fwd_kernel(log2n), dft_smem(log2n));
+  if (cudaSuccess == e) e = raise_smem_limit(dft_fwd_rhs_kernel(log2n), dft_smem(log2n));
+  if (cudaSuccess == e) e = raise_smem_limit(dft_inv_kernel(log2n), dft_smem(log2n));
+  if (cudaSuccess == e) e = svof_cline::cline_prepare<double>((1L << log2n) / 2 + 1, nx);
+  return e;
+}
+cudaError_t dft_pivots(cudaStream_t st, double *tab, const double *pl, const double *pu, const double *evals, int nx,
+                       int nky) {
+  using namespace svof_cline;
+  k_cline_table<<<(nky + kTabLines - 1) / kTabLines, kTabLines, 0, st>>>(tab, pl, pu, evals, nullptr, nky, nky, nx,
+                                                                        nullptr);
+  return cudaGetLastError();
 }
 
 }  // namespace svof

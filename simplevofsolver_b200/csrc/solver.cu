@@ -16,6 +16,7 @@
 #include <cstdlib>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <map>
 #include <string>
 #include <vector>
@@ -249,7 +250,8 @@ int launch_predict(svof_solver *s, int rk, bool with_coef) {
   return 0;
 }
 
-int launch_potential(svof_solver *s, int rk, int want_dct) {
+int launch_potential(svof_solver *s, int rk, int want_dct, const std::function<int(int)> &mark) {
+  auto m = [&](int kind) { return mark ? mark(kind) : 0; };
   const double gam = RK_A[rk] + RK_B[rk];
   const Grid2 g = s->grid();
   if (want_dct != (int)s->uniform) {
@@ -261,23 +263,29 @@ int launch_potential(svof_solver *s, int rk, int want_dct) {
     CK(launch_k(s->pdl, dct_fwd_kernel(L), rows_grid, dct_threads(L), dct_smem(L, false), s->stream,
                 (const double *)s->ux[s->cur_u].p, (const double *)s->uy[s->cur_u].p, s->spec.p,
                 (const double *)s->twf.p, (const double *)s->cs.p, (const double *)s->d_dt, gam, g));
+    if (m(SVOF_K_POISSON_FWD)) return 1;
     const int kt = s->ysolve_kt;
     CK(launch_k(s->pdl, k_dct_ysolve, (s->nx + kt - 1) / kt, 128, sizeof(double) * 3 * kt * s->ny, s->stream,
                 s->spec.p, s->vt.p, s->rvt.p, s->q1t.p, s->ck.p, s->lastf.p, s->den.p, 1. / s->dy / s->dy, s->nx,
                 s->ny, kt));
+    if (m(SVOF_K_POISSON_SOLVE)) return 1;
     CK(launch_k(s->pdl, dct_inv_kernel(L), rows_grid, dct_threads(L), dct_smem(L, true), s->stream,
                 (const double *)s->spec.p, s->psi.p, (const double *)s->twb.p, (const double *)s->cs.p, g));
+    if (m(SVOF_K_POISSON_INV)) return 1;
   } else {
-    const int cols = s->dft_cols;
-    const int blocks = (s->nx + cols - 1) / cols;
-    const size_t smem = sizeof(double) * 2 * s->ny * cols;
-    const int nky = s->ny / 2 + 1;
-    CK(launch_k(s->pdl, k_dft_fwd, blocks, 256, smem, s->stream, s->ux[s->cur_u].p, s->uy[s->cur_u].p, s->spec.p,
-                s->twf.p, s->d_dt, gam, s->log2fft, cols, g));
-    const int xkt = s->xsolve_kt;
-    CK(launch_k(s->pdl, k_dft_xsolve, (nky + xkt - 1) / xkt, 128, sizeof(double) * 4 * xkt * s->nx, s->stream,
-                s->spec.p, s->vt.p, s->rvt.p, s->pl.p, s->pu.p, s->evals.p, s->nx, nky, xkt));
-    CK(launch_k(s->pdl, k_dft_inv, blocks, 256, smem, s->stream, s->spec.p, s->psi.p, s->twb.p, s->log2fft, cols, g));
+    const int L = s->log2fft, nky = s->ny / 2 + 1, lpb = dft_xsolve_lines(nky, s->nx);
+    const dim3 cols_grid((s->nx + dft_cols(L) - 1) / dft_cols(L));
+    CK(launch_k(s->pdl, dft_fwd_kernel(L), cols_grid, dft_threads(L), dft_smem(L), s->stream,
+                (const double *)s->ux[s->cur_u].p, (const double *)s->uy[s->cur_u].p, s->spec.p,
+                (const double *)s->twf.p, (const double *)s->d_dt, gam, g));
+    if (m(SVOF_K_POISSON_FWD)) return 1;
+    CK(launch_k(s->pdl, dft_xsolve_kernel(nky, s->nx), (nky + lpb - 1) / lpb, 32, dft_xsolve_smem(nky, s->nx),
+                s->stream, s->spec.p, (const double *)s->rvt.p, (const double *)s->pl.p, (const double *)s->pu.p,
+                (long)nky, s->nx, 0, (unsigned long long *)nullptr, (const unsigned long long *)nullptr));
+    if (m(SVOF_K_POISSON_SOLVE)) return 1;
+    CK(launch_k(s->pdl, dft_inv_kernel(L), cols_grid, dft_threads(L), dft_smem(L), s->stream,
+                (const double *)s->spec.p, s->psi.p, (const double *)s->twb.p, g));
+    if (m(SVOF_K_POISSON_INV)) return 1;
   }
   return 0;
 }
@@ -488,7 +496,7 @@ int build_tables(svof_solver *s, const double *xf, const double *xc) {
   } else {
     // src/fluid/compute_potential/dft.c:142-198 and :263-291
     const int n = nx, nky = ny / 2 + 1;
-    std::vector<double> pl(n), pu(n), ev(nky), c(n), v(n), vt((size_t)n * nky, 0.), rvt((size_t)n * nky, 0.);
+    std::vector<double> pl(n), pu(n), ev(nky);
     for (int i = 1; i <= n; i++) {
       pl[i - 1] = 1. / DXC(i) / DXF(i);
       pu[i - 1] = 1. / DXC(i + 1) / DXF(i);
@@ -498,21 +506,9 @@ int build_tables(svof_solver *s, const double *xf, const double *xc) {
     for (size_t j = 0; j < (size_t)nky; j++) {
       ev[j] = -4. / std::pow(gridsize, 2.) * std::pow(std::sin(kGPi * j / signal_length), 2.);
     }
-    for (int k = 0; k < nky; k++) {
-      for (int i = 0; i < n; i++) c[i] = -pl[i] - pu[i] + ev[k];
-      c[0] += pl[0];
-      c[n - 1] += pu[n - 1];
-      v[0] = pu[0] / c[0];
-      for (int i = 1; i < n - 1; i++) {
-        const double val = 1. / (c[i] - pl[i] * v[i - 1]);
-        v[i] = val * (pu[i]);
-        rvt[(size_t)i * nky + k] = val;
-      }
-      for (int i = 0; i < n - 1; i++) vt[(size_t)i * nky + k] = v[i];
-    }
-    if (upload(s->pl, pl) || upload(s->pu, pu) || upload(s->evals, ev) || upload(s->vt, vt) ||
-        upload(s->rvt, rvt))
-      return 1;
+    if (upload(s->pl, pl) || upload(s->pu, pu) || upload(s->evals, ev) || dalloc(s->rvt, (size_t)n * nky)) return 1;
+    CK(cudaDeviceSynchronize());
+    CK(dft_pivots(s->stream, s->rvt.p, s->pl.p, s->pu.p, s->evals.p, n, nky));
     if (dalloc(s->spec, 2 * (size_t)nx * nky)) return 1;
   }
   return 0;
@@ -614,15 +610,10 @@ int engine_create(const svof_params_t *prm, const double *xf, const double *xc, 
       return fail("svof_create: the DCT path takes nx = 4 .. 4096 (got %d)", nx), bail();
     if (s->uniform && cudaSuccess != dct_prepare(s->log2fft))
       return fail("cudaFuncSetAttribute(k_dct_fwd, k_dct_inv)"), bail();
-    int cols = 16;
-    while (cols > 1 && sizeof(double) * 2 * (size_t)ny * cols > 100 * 1024) cols >>= 1;
-    s->dft_cols = cols;
-    const size_t dft_smem = sizeof(double) * 2 * (size_t)ny * cols;
-    if (!s->uniform && (cudaSuccess != raise_smem_limit(k_dft_fwd, dft_smem) ||
-                        cudaSuccess != raise_smem_limit(k_dft_inv, dft_smem)))
-      return fail("cudaFuncSetAttribute(k_dft_fwd, k_dft_inv)"), bail();
-    if (!s->uniform && sizeof(double) * 2 * (size_t)ny > 200 * 1024)
-      return fail("svof_create: FFT length too large for one block"), bail();
+    if (!s->uniform && !dft_length_ok(s->log2fft))
+      return fail("svof_create: the DFT path takes ny = 4 .. 8192 (got %d)", ny), bail();
+    if (!s->uniform && cudaSuccess != dft_prepare(s->log2fft, nx))
+      return fail("cudaFuncSetAttribute(k_dft_fwd, k_dft_inv, k_cline_solve)"), bail();
   }
   // line solves: lines per block so that there are four blocks per SM where
   // the lines allow (one block's staging overlaps the others' sweeps), within
@@ -639,12 +630,6 @@ int engine_create(const svof_params_t *prm, const double *xf, const double *xc, 
     const size_t sm = bpl * s->ysolve_kt;
     if (sm > 200 * 1024) return fail("svof_create: ny = %d too large for the y line solver", ny), bail();
     if (cudaSuccess != raise_smem_limit(k_dct_ysolve, sm)) return fail("cudaFuncSetAttribute(k_dct_ysolve)"), bail();
-  } else {
-    const size_t bpl = sizeof(double) * 4 * (size_t)nx;
-    s->xsolve_kt = pick_kt(ny / 2 + 1, bpl);
-    const size_t sm = bpl * s->xsolve_kt;
-    if (sm > 200 * 1024) return fail("svof_create: nx = %d too large for the x line solver", nx), bail();
-    if (cudaSuccess != raise_smem_limit(k_dft_xsolve, sm)) return fail("cudaFuncSetAttribute(k_dft_xsolve)"), bail();
   }
   // launch plan checks: every dynamic shared-memory size covers what the
   // kernel indexes, every line solve has a thread per line
@@ -654,8 +639,6 @@ int engine_create(const svof_params_t *prm, const double *xf, const double *xc, 
       return fail("svof_create: inconsistent predictor launch plan"), bail();
     if (s->uniform && (s->ysolve_kt < 1 || s->ysolve_kt > 64 || s->ysolve_kt > 128))
       return fail("svof_create: inconsistent y line-solve launch plan"), bail();
-    if (!s->uniform && (s->xsolve_kt < 1 || s->xsolve_kt > 128 || s->dft_cols < 1))
-      return fail("svof_create: inconsistent x line-solve launch plan"), bail();
   }
   if (cudaSuccess != cudaMalloc(&s->d_dt, sizeof(double))) return fail("cudaMalloc dt"), bail();
   if (cudaSuccess != cudaMalloc(&s->d_minbits, sizeof(unsigned long long))) return fail("cudaMalloc"), bail();
@@ -968,40 +951,7 @@ int svof_profile_step(svof_solver_t *s, double *ms, int *launches, int nkinds) {
     rc = rc || launch_force(s) || mark(SVOF_K_FORCE);
     rc = rc || launch_vof(s, rk) || mark(SVOF_K_VOF);
     rc = rc || launch_predict(s, rk) || mark(SVOF_K_PREDICT);
-    if (!rc) {
-      const double gam = RK_A[rk] + RK_B[rk];
-      const Grid2 g = s->grid();
-      if (s->uniform) {
-        const int L = s->log2fft;
-        const dim3 rows_grid((s->ny + dct_rows(L) - 1) / dct_rows(L));
-        dct_fwd_kernel(L)<<<rows_grid, dct_threads(L), dct_smem(L, false), s->stream>>>(
-            s->ux[s->cur_u].p, s->uy[s->cur_u].p, s->spec.p, s->twf.p, s->cs.p, s->d_dt, gam, g);
-        rc = rc || mark(SVOF_K_POISSON_FWD);
-        const int kt = s->ysolve_kt;
-        k_dct_ysolve<<<(s->nx + kt - 1) / kt, 128, sizeof(double) * 3 * kt * s->ny, s->stream>>>(
-            s->spec.p, s->vt.p, s->rvt.p, s->q1t.p, s->ck.p, s->lastf.p, s->den.p, 1. / s->dy / s->dy, s->nx,
-            s->ny, kt);
-        rc = rc || mark(SVOF_K_POISSON_SOLVE);
-        dct_inv_kernel(L)<<<rows_grid, dct_threads(L), dct_smem(L, true), s->stream>>>(s->spec.p, s->psi.p, s->twb.p,
-                                                                                     s->cs.p, g);
-        rc = rc || mark(SVOF_K_POISSON_INV);
-      } else {
-        const int cols = s->dft_cols;
-        const int blocks = (s->nx + cols - 1) / cols;
-        const size_t smem = sizeof(double) * 2 * s->ny * cols;
-        const int nky = s->ny / 2 + 1;
-        k_dft_fwd<<<blocks, 256, smem, s->stream>>>(s->ux[s->cur_u].p, s->uy[s->cur_u].p, s->spec.p, s->twf.p,
-                                                    s->d_dt, gam, s->log2fft, cols, g);
-        rc = rc || mark(SVOF_K_POISSON_FWD);
-        const int xkt = s->xsolve_kt;
-        k_dft_xsolve<<<(nky + xkt - 1) / xkt, 128, sizeof(double) * 4 * xkt * s->nx, s->stream>>>(
-            s->spec.p, s->vt.p, s->rvt.p, s->pl.p, s->pu.p, s->evals.p, s->nx, nky, xkt);
-        rc = rc || mark(SVOF_K_POISSON_SOLVE);
-        k_dft_inv<<<blocks, 256, smem, s->stream>>>(s->spec.p, s->psi.p, s->twb.p, s->log2fft, cols, g);
-        rc = rc || mark(SVOF_K_POISSON_INV);
-      }
-      rc = rc || (cudaSuccess != cudaGetLastError());
-    }
+    rc = rc || launch_potential(s, rk, s->uniform, mark);
     rc = rc || launch_project(s, rk, 1, 1) || mark(SVOF_K_PROJECT);
   }
   cudaError_t e = cudaStreamSynchronize(s->stream);

@@ -3,6 +3,7 @@
 // adjoint.cu (the differentiation form).
 #pragma once
 
+#include <functional>
 #include <cuda_runtime.h>
 
 #include <map>
@@ -65,8 +66,6 @@ struct svof_solver {
   int pred_rows = 1;
   int pred_threads = 256;
   size_t pred_smem = 0;
-  int xsolve_kt = 8;        // ky lines per block of the DFT x solve
-  int dft_cols = 1;
   // time step
   double *d_dt = nullptr;
   unsigned long long *d_minbits = nullptr;
@@ -155,7 +154,8 @@ int launch_force(svof_solver *s, cudaStream_t st = nullptr);
 int launch_vof(svof_solver *s, int rk);
 // with_coef: launch k_tdm_coef first on the same stream
 int launch_predict(svof_solver *s, int rk, bool with_coef = true);
-int launch_potential(svof_solver *s, int rk, int want_dct);
+// (`mark`, may be empty, is called with the kernel kind after each launch)
+int launch_potential(svof_solver *s, int rk, int want_dct, const std::function<int(int)> &mark = {});
 int launch_project(svof_solver *s, int rk, int do_vel, int do_p);
 
 // frees the differentiation form's buffers (adjoint.cu)

@@ -141,22 +141,33 @@ __global__ void k_dct_ysolve(double *__restrict__ spec, const double *__restrict
                              const double *__restrict__ rvt, const double *__restrict__ q1t,
                              const double *__restrict__ ck, const double *__restrict__ lastf,
                              const double *__restrict__ den, double lap, int nx, int ny, int kt);
-// Poisson, DFT path (src/fluid/compute_potential/dft.c)
-__global__ void k_dft_fwd(const double *__restrict__ ux, const double *__restrict__ uy,
-                          double *__restrict__ spec, const double *__restrict__ tw,
-                          const double *__restrict__ dtp, double gam, int log2n, int cols, Grid2 g);
-__global__ void k_dft_xsolve(double *__restrict__ spec, const double *__restrict__ vt,
-                             const double *__restrict__ rvt, const double *__restrict__ pl,
-                             const double *__restrict__ pu, const double *__restrict__ evals, int nx,
-                             int nky, int kt);
-__global__ void k_dft_inv(const double *__restrict__ spec, double *__restrict__ psi,
-                          const double *__restrict__ tw, int log2n, int cols, Grid2 g);
-
-// the DFT path's forward transform on a right-hand side r[j-1][i-1] /
-// dxf[i-1] (the adjoint's second Poisson solve, with the grid-metric weights
-// of the x grid); k_dft_fwd's launch shape
-__global__ void k_dft_fwd_rhs(const double *__restrict__ r, double *__restrict__ spec, const double *__restrict__ tw,
-                              int log2n, int cols, Grid2 g);
+// Poisson, DFT path (src/fluid/compute_potential/dft.c).  The column
+// transforms (k_dft_fwd: divergence right-hand side + r2c along y;
+// k_dft_fwd_rhs: the same on an array right-hand side r[j-1][i-1] /
+// dxf[i-1], the adjoint's second solve; k_dft_inv: c2r + psi columns with halo
+// and walls) are compiled per length ny = 2^log2n, log2n in [kDctMinL2N,
+// kDftMaxL2N]: dft_threads(log2n) threads, dft_cols(log2n) columns per block,
+// dft_smem(log2n) bytes; the x solves (cline_solve.cuh): one warp per
+// dft_xsolve_lines lines, on the pivots that dft_pivots makes (nx per line).
+constexpr int kDftMaxL2N = 13;
+using DftFwdKernel = void (*)(const double *, const double *, double *, const double *, const double *, double, Grid2);
+using DftFwdRhsKernel = void (*)(const double *, double *, const double *, Grid2);
+using DftInvKernel = void (*)(const double *, double *, const double *, Grid2);
+using DftXSolveKernel = void (*)(double *, const double *, const double *, const double *, long, int, int,
+                                 unsigned long long *, const unsigned long long *);
+bool dft_length_ok(int log2n);
+int dft_cols(int log2n);
+int dft_threads(int log2n);
+size_t dft_smem(int log2n);
+DftFwdKernel dft_fwd_kernel(int log2n);
+DftFwdRhsKernel dft_fwd_rhs_kernel(int log2n);
+DftInvKernel dft_inv_kernel(int log2n);
+DftXSolveKernel dft_xsolve_kernel(long nlines, int nx);
+int dft_xsolve_lines(long nlines, int nx);
+size_t dft_xsolve_smem(long nlines, int nx);
+cudaError_t dft_prepare(int log2n, int nx);
+cudaError_t dft_pivots(cudaStream_t st, double *tab, const double *pl, const double *pu, const double *evals, int nx,
+                       int nky);
 
 // projection and pressure update, in place (src/fluid/correct_velocity/*.c,
 // src/fluid/update_pressure.c); do_vel / do_p select the two halves
