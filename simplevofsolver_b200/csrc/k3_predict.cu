@@ -25,6 +25,7 @@
 
 #include "svof3d_internal.cuh"
 #include "smem_limit.cuh"
+#include "tdm_pivots.cuh"
 
 // Precision split as in k3_interface.cu: SVOF3_PRECISION=64 builds the FP64
 // instantiations and the shared code (no FMA contraction), =32 the FP32
@@ -50,12 +51,13 @@ __global__ void k3_tdm_coef(const double *__restrict__ lap_ux, const double *__r
                             const double *__restrict__ dtp, double gam, double m_dif, double t_dif, int nx,
                             double *__restrict__ coef) {
   extern __shared__ double slap[];  // [2][3 nx]
+#pragma unroll 4
   for (int w = threadIdx.x; w < 3 * nx; w += blockDim.x) {
     slap[w] = (w < 3 * (nx - 1)) ? lap_ux[w] : 0.;
     slap[3 * nx + w] = lap_cc[w];
   }
   __syncthreads();
-  const int f = threadIdx.x;
+  const int f = threadIdx.x >> 5;  // a warp a system
   if (f >= 3) return;
   const double *lap = slap + ((0 == f) ? 0 : 3 * nx);
   const double dif = (2 == f) ? t_dif : m_dif;
@@ -63,30 +65,8 @@ __global__ void k3_tdm_coef(const double *__restrict__ lap_ux, const double *__r
   double *L = coef + (size_t)(3 * f + 0) * nx;
   double *R = coef + (size_t)(3 * f + 1) * nx;
   double *V = coef + (size_t)(3 * f + 2) * nx;
-  const double dt = *dtp;
-  const double pf = 0.5 * gam * dt * dif;
-  const double c0 = 1. - pf * lap[1];
-  double v = (-pf * lap[2]) / c0;
-  L[0] = -pf * lap[0];
-  R[0] = c0;
-  V[0] = v;
-  for (int i = 1; i < n - 1; i++) {
-    const double l = -pf * lap[3 * i + 0];
-    const double c = 1. - pf * lap[3 * i + 1];
-    const double u = -pf * lap[3 * i + 2];
-    const double val = 1. / (c - l * v);
-    v = val * (u);
-    L[i] = l;
-    R[i] = val;
-    V[i] = v;
-  }
-  {
-    const double l = -pf * lap[3 * (n - 1) + 0];
-    const double c = 1. - pf * lap[3 * (n - 1) + 1];
-    const double val = c - l * v;
-    L[n - 1] = l;
-    R[n - 1] = fabs(val) > kDblEpsilon ? 1. / val : 0.;
-  }
+  const double pf = 0.5 * gam * *dtp * dif;
+  svof_tdm::pivots(lap, pf, n, L, R, V);
 }
 #endif
 

@@ -14,6 +14,7 @@
 #include <cuda_pipeline.h>
 
 #include "svof_internal.cuh"
+#include "tdm_pivots.cuh"
 
 namespace svof {
 
@@ -24,8 +25,8 @@ size_t predict_smem_bytes(int nx, int R) {
 
 // Thomas coefficients of the three implicit-x systems of one substep
 // (solve_in_x of src/fluid/predict/{ux,uy,t}.c and gtsv, src/tdm.c:17-50):
-// they depend on dt and the substep only, so one thread per field computes
-// them once and every line solve reads them.  Layout per field f at
+// they depend on dt and the substep only, so one warp per field computes
+// them once (tdm_pivots.cuh) and every line solve reads them.  Layout per field f at
 // coef + 3 f nx:  L[i] = tdm_l[i];  R[0] = tdm_c[0], R[i] = 1 / (c_i - l_i
 // v_{i-1}) for 0 < i < n-1, R[n-1] = 1 / (c - l v) of the last row or 0 when
 // the reference zeroes that row;  V[i] = v_i.
@@ -39,13 +40,14 @@ __global__ void k_tdm_coef(const double *__restrict__ lap_ux, const double *__re
   // the Laplacian tables are staged in shared memory first: the recurrence
   // below then waits on arithmetic only
   extern __shared__ double slap[];  // [3][3 nx]
+#pragma unroll 4
   for (int w = threadIdx.x; w < 3 * nx; w += blockDim.x) {
     slap[w] = (w < 3 * (nx - 1)) ? lap_ux[w] : 0.;
     slap[3 * nx + w] = lap_uy[w];
     slap[6 * nx + w] = lap_t[w];
   }
   __syncthreads();
-  const int f = threadIdx.x;
+  const int f = threadIdx.x >> 5;  // a warp a system
   if (f >= 3) return;
   const double *lap = slap + 3 * nx * f;
   const double dif = (2 == f) ? t_dif : m_dif;
@@ -53,30 +55,8 @@ __global__ void k_tdm_coef(const double *__restrict__ lap_ux, const double *__re
   double *L = coef + (size_t)(3 * f + 0) * nx;
   double *R = coef + (size_t)(3 * f + 1) * nx;
   double *V = coef + (size_t)(3 * f + 2) * nx;
-  const double dt = *dtp;
-  const double pf = 0.5 * gam * dt * dif;  // ux.c:330-332
-  const double c0 = 1. - pf * lap[1];
-  double v = (-pf * lap[2]) / c0;
-  L[0] = -pf * lap[0];
-  R[0] = c0;
-  V[0] = v;
-  for (int i = 1; i < n - 1; i++) {
-    const double l = -pf * lap[3 * i + 0];
-    const double c = 1. - pf * lap[3 * i + 1];
-    const double u = -pf * lap[3 * i + 2];
-    const double val = 1. / (c - l * v);
-    v = val * (u);
-    L[i] = l;
-    R[i] = val;
-    V[i] = v;
-  }
-  {
-    const double l = -pf * lap[3 * (n - 1) + 0];
-    const double c = 1. - pf * lap[3 * (n - 1) + 1];
-    const double val = c - l * v;
-    L[n - 1] = l;
-    R[n - 1] = fabs(val) > kDblEpsilon ? 1. / val : 0.;
-  }
+  const double pf = 0.5 * gam * *dtp * dif;  // ux.c:330-332
+  svof_tdm::pivots(lap, pf, n, L, R, V);
 }
 
 // right-hand sides of ux (i >= 2), uy and t at cell (i, j), exactly as

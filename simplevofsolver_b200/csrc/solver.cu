@@ -177,7 +177,7 @@ double *coef_table(svof_solver *s, int rk) { return s->coef.p + (size_t)9 * s->n
 
 int launch_coef(svof_solver *s, int rk, cudaStream_t st) {
   Gam3 g{{RK_A[rk] + RK_B[rk], 0., 0.}};
-  CK(launch_k(s->pdl, k_tdm_coef, 1, 128, sizeof(double) * 9 * s->nx, st, (const double *)s->lap_ux.p,
+  CK(launch_k(s->pdl, k_tdm_coef, 1, 256, sizeof(double) * 9 * s->nx, st, (const double *)s->lap_ux.p,
               (const double *)s->lap_uy.p, (const double *)s->lap_t.p, (const double *)s->d_dt, g, s->prm.m_dif,
               s->prm.t_dif, s->nx, coef_table(s, rk)));
   return 0;
@@ -186,7 +186,7 @@ int launch_coef(svof_solver *s, int rk, cudaStream_t st) {
 // the three substeps' tables at once (they need only dt), one block each
 int launch_coef_all(svof_solver *s, cudaStream_t st) {
   Gam3 g{{RK_A[0] + RK_B[0], RK_A[1] + RK_B[1], RK_A[2] + RK_B[2]}};
-  CK(launch_k(s->pdl, k_tdm_coef, 3, 128, sizeof(double) * 9 * s->nx, st, (const double *)s->lap_ux.p,
+  CK(launch_k(s->pdl, k_tdm_coef, 3, 256, sizeof(double) * 9 * s->nx, st, (const double *)s->lap_ux.p,
               (const double *)s->lap_uy.p, (const double *)s->lap_t.p, (const double *)s->d_dt, g, s->prm.m_dif,
               s->prm.t_dif, s->nx, coef_table(s, 0)));
   return 0;

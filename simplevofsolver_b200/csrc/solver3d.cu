@@ -293,7 +293,7 @@ int launch_predict_t(svof3d_solver *s, int rk) {
 }
 
 int launch_predict(svof3d_solver *s, int rk) {
-  k3_tdm_coef<<<1, 128, sizeof(double) * 6 * s->nx, s->stream>>>(s->lap_ux.p, s->lap_cc.p, s->d_dt,
+  k3_tdm_coef<<<1, 256, sizeof(double) * 6 * s->nx, s->stream>>>(s->lap_ux.p, s->lap_cc.p, s->d_dt,
                                                                  RK_A[rk] + RK_B[rk], s->prm.m_dif, s->prm.t_dif,
                                                                  s->nx, s->coef.p);
   CK_LAUNCH();
@@ -1324,7 +1324,7 @@ template <class S>
 int adj3_predict_t(svof3d_solver *s, int rk, double dt, const double *ux, const double *uy, const double *uz,
                    const double *vof_post) {
   Adjoint3State *a = s->adj;
-  k3_tdm_coef<<<1, 128, sizeof(double) * 6 * s->nx, s->stream>>>(s->lap_ux.p, s->lap_cc.p, s->d_dt,
+  k3_tdm_coef<<<1, 256, sizeof(double) * 6 * s->nx, s->stream>>>(s->lap_ux.p, s->lap_cc.p, s->d_dt,
                                                                  RK_A[rk] + RK_B[rk], s->prm.m_dif, s->prm.t_dif,
                                                                  s->nx, s->coef.p);
   CK_LAUNCH();
