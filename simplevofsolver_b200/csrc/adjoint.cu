@@ -278,18 +278,18 @@ int svof_integrate_fixed(svof_solver_t *s, double dt, double *tape) {
   if (adj_set_dt(s, dt)) return 1;
   const size_t n_ux = (size_t)(s->nx + 1) * (s->ny + 2), n_cc = (size_t)(s->nx + 2) * (s->ny + 2);
   const size_t n_vof = (size_t)(s->nx + 2) * (s->ny + 4), st = tape_stride(s);
-  for (int rk = 0; rk < 3; rk++) {
-    if (tape) {
-      double *t = tape + rk * st;
-      CK(cudaMemcpyAsync(t, s->ux[s->cur_u].p, sizeof(double) * n_ux, cudaMemcpyDeviceToDevice, s->stream));
-      CK(cudaMemcpyAsync(t + n_ux, s->uy[s->cur_u].p, sizeof(double) * n_cc, cudaMemcpyDeviceToDevice, s->stream));
+  auto record = [&](int rk, cudaStream_t stream, bool interface) -> int {
+    double *t = tape + rk * st;
+    if (interface) {
       CK(cudaMemcpyAsync(t + n_ux + n_cc, s->vof[s->cur_v].p, sizeof(double) * n_vof, cudaMemcpyDeviceToDevice,
-                         s->stream));
+                         stream));
+    } else {
+      CK(cudaMemcpyAsync(t, s->ux[s->cur_u].p, sizeof(double) * n_ux, cudaMemcpyDeviceToDevice, stream));
+      CK(cudaMemcpyAsync(t + n_ux, s->uy[s->cur_u].p, sizeof(double) * n_cc, cudaMemcpyDeviceToDevice, stream));
     }
-    if (launch_coef(s, rk, s->stream) || launch_geom(s) || launch_force(s) || launch_vof(s, rk) ||
-        launch_predict(s, rk, false) || launch_potential(s, rk, s->uniform) || launch_project(s, rk, 1, 1))
-      return 1;
-  }
+    return 0;
+  };
+  if (tape ? launch_substeps(s, false, record) : launch_substeps(s, false, {})) return 1;
   if (tape)
     CK(cudaMemcpyAsync(tape + 3 * st, s->vof[s->cur_v].p, sizeof(double) * n_vof, cudaMemcpyDeviceToDevice,
                        s->stream));

@@ -147,9 +147,9 @@ int launch_dt(svof_solver *s) {
   return 0;
 }
 
-int launch_geom(svof_solver *s) {
+int launch_geom(svof_solver *s, cudaStream_t st) {
   dim3 b(32, 8), gr((s->nx + 31) / 32, (s->ny + 2 + 7) / 8);
-  CK(launch_k(s->pdl, k_geom, gr, b, 0, s->stream, (const double *)s->vof[s->cur_v].p, s->normal.p, s->curv.p,
+  CK(launch_k(s->pdl, k_geom, gr, b, 0, st ? st : s->stream, (const double *)s->vof[s->cur_v].p, s->normal.p, s->curv.p,
               s->grid()));
   return 0;
 }
@@ -161,11 +161,11 @@ int launch_force(svof_solver *s, cudaStream_t st) {
   return 0;
 }
 
-int launch_vof(svof_solver *s, int rk) {
+int launch_vof(svof_solver *s, int rk, cudaStream_t st) {
   if (0 != rk) s->sa_v ^= 1;  // reset_srcs, src/interface/update/main.c:28-45
   dim3 b(32, 8), gr((s->nx + 31) / 32, (s->ny + 7) / 8);
   RK c{RK_A[rk], RK_B[rk], RK_A[rk] + RK_B[rk]};
-  CK(launch_k(s->pdl, k_vof_advect, gr, b, 0, s->stream, (const double *)s->vof[s->cur_v].p, s->vof[1 - s->cur_v].p,
+  CK(launch_k(s->pdl, k_vof_advect, gr, b, 0, st ? st : s->stream, (const double *)s->vof[s->cur_v].p, s->vof[1 - s->cur_v].p,
               (const double *)s->ux[s->cur_u].p, (const double *)s->uy[s->cur_u].p, (const double *)s->normal.p,
               s->svof[s->sa_v].p, (const double *)s->svof[1 - s->sa_v].p, (const double *)s->d_dt, c, rk != 0,
               s->grid()));
@@ -298,33 +298,58 @@ int launch_project(svof_solver *s, int rk, int do_vel, int do_p) {
   return 0;
 }
 
-// the kernel sequence of integrate(), src/integrate.c:11-68
-int launch_step(svof_solver *s) {
-  if (launch_dt(s)) return 1;
-  // the three substeps' predictor coefficients need only dt: one launch on a
-  // branch of its own, beside the first substep's interface kernels (the
-  // serial recurrence takes about as long as they do)
-  CK(cudaEventRecord(s->ev_fork[0], s->stream));
-  CK(cudaStreamWaitEvent(s->side2, s->ev_fork[0], 0));
+// The three substeps of integrate(), src/integrate.c:24-65, after the time
+// step is known (with_dt: computed here).  Two branches: the interface's
+// kernels (geometry, force and vof advection) need the fluid only where the
+// advection reads a substep's corrected velocity, the fluid's only the force,
+// so the geometry and force of substep k + 1 and the advection of substep k
+// run beside the predictor, the Poisson solve and the projection of substep
+// k, whose line solves leave most of the chip idle.  Waits between the
+// branches: the advection for the previous projection, the predictor for its
+// force (and for the advected vof where that is buoyant), the next force for
+// the predictor that still reads this one's arrays.  The three substeps'
+// predictor coefficients need dt alone and have a branch of their own.
+// us a step, against the force beside the advection and the rest in line:
+// 32^2 153 -> 130, 128^2 153 -> 130, stretched 128 x 256 200 -> 170, 1024^2
+// 1048 -> 1018; the fixed steps of a 256^2 gradient 24.0 -> 21.5 ms a pass.
+// tape (may be empty): called with (substep, stream, the interface's branch)
+// where the branch holds that substep's inputs
+int launch_substeps(svof_solver *s, bool with_dt, const std::function<int(int, cudaStream_t, bool)> &tape) {
+  CK(cudaEventRecord(s->ev_fork, s->stream));
+  CK(cudaStreamWaitEvent(s->side, s->ev_fork, 0));
+  if (launch_geom(s, s->side) || launch_force(s, s->side)) return 1;
+  CK(cudaEventRecord(s->ev_force[0], s->side));
+  if (with_dt && launch_dt(s)) return 1;
+  CK(cudaEventRecord(s->ev_dt, s->stream));
+  CK(cudaStreamWaitEvent(s->side2, s->ev_dt, 0));
   if (launch_coef_all(s, s->side2)) return 1;
   CK(cudaEventRecord(s->ev_coef, s->side2));
+  CK(cudaStreamWaitEvent(s->side, s->ev_dt, 0));
   for (int rk = 0; rk < 3; rk++) {
-    if (launch_geom(s)) return 1;
-    // the CSF force and the vof advection both only need the geometry: the
-    // force runs beside the advection, on the side branch
-    CK(cudaEventRecord(s->ev_geom[rk], s->stream));
-    CK(cudaStreamWaitEvent(s->side, s->ev_geom[rk], 0));
-    if (launch_force(s, s->side)) return 1;
-    CK(cudaEventRecord(s->ev_join[rk], s->side));
-    if (launch_vof(s, rk)) return 1;
-    CK(cudaStreamWaitEvent(s->stream, s->ev_join[rk], 0));
+    if (rk > 0) CK(cudaStreamWaitEvent(s->side, s->ev_project[rk - 1], 0));
+    if (tape && (tape(rk, s->side, true) || tape(rk, s->stream, false))) return 1;
+    if (launch_vof(s, rk, s->side)) return 1;
+    CK(cudaEventRecord(s->ev_vof[rk], s->side));
+    if (rk < 2 && launch_geom(s, s->side)) return 1;
+    CK(cudaStreamWaitEvent(s->stream, s->ev_force[rk], 0));
     if (0 == rk) CK(cudaStreamWaitEvent(s->stream, s->ev_coef, 0));
+    if (0. != s->grav_vof) CK(cudaStreamWaitEvent(s->stream, s->ev_vof[rk], 0));
     if (launch_predict(s, rk, false)) return 1;
-    if (launch_potential(s, rk, s->uniform)) return 1;
-    if (launch_project(s, rk, 1, 1)) return 1;
+    if (rk < 2) {
+      CK(cudaEventRecord(s->ev_predict[rk], s->stream));
+      CK(cudaStreamWaitEvent(s->side, s->ev_predict[rk], 0));
+      if (launch_force(s, s->side)) return 1;
+      CK(cudaEventRecord(s->ev_force[rk + 1], s->side));
+    }
+    if (launch_potential(s, rk, s->uniform) || launch_project(s, rk, 1, 1)) return 1;
+    if (rk < 2) CK(cudaEventRecord(s->ev_project[rk], s->stream));
   }
+  CK(cudaStreamWaitEvent(s->stream, s->ev_vof[2], 0));
   return 0;
 }
+
+// the kernel sequence of integrate(), src/integrate.c:11-68
+int launch_step(svof_solver *s) { return launch_substeps(s, true, {}); }
 
 int state_key(const svof_solver *s) { return s->cur_u | (s->cur_v << 1) | (s->sa_f << 2) | (s->sa_v << 3); }
 
@@ -571,13 +596,8 @@ int engine_create(const svof_params_t *prm, const double *xf, const double *xc, 
   if (dalloc(s->coef, 27 * (size_t)nx)) return bail();  // one table per substep
   if (cudaSuccess != cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking)) return fail("stream"), bail();
   if (cudaSuccess != cudaStreamCreateWithFlags(&s->side2, cudaStreamNonBlocking)) return fail("stream"), bail();
-  if (cudaSuccess != cudaEventCreateWithFlags(&s->ev_coef, cudaEventDisableTiming)) return fail("event"), bail();
-  for (int k = 0; k < 3; k++) {
-    if (cudaSuccess != cudaEventCreateWithFlags(&s->ev_fork[k], cudaEventDisableTiming) ||
-        cudaSuccess != cudaEventCreateWithFlags(&s->ev_geom[k], cudaEventDisableTiming) ||
-        cudaSuccess != cudaEventCreateWithFlags(&s->ev_join[k], cudaEventDisableTiming))
-      return fail("event"), bail();
-  }
+  for (cudaEvent_t *e : s->branch_events())
+    if (cudaSuccess != cudaEventCreateWithFlags(e, cudaEventDisableTiming)) return fail("event"), bail();
   // predict launch shape: R rows per block, enough blocks to cover the SMs,
   // within 200 KB of shared memory
   {
@@ -709,12 +729,8 @@ int svof_destroy(svof_solver_t *s) {
   if (s->d_minbits) cudaFree(s->d_minbits);
   if (s->d_status) cudaFree(s->d_status);
   if (s->h_dt) cudaFreeHost(s->h_dt);
-  for (int k = 0; k < 3; k++) {
-    if (s->ev_fork[k]) cudaEventDestroy(s->ev_fork[k]);
-    if (s->ev_geom[k]) cudaEventDestroy(s->ev_geom[k]);
-    if (s->ev_join[k]) cudaEventDestroy(s->ev_join[k]);
-  }
-  if (s->ev_coef) cudaEventDestroy(s->ev_coef);
+  for (cudaEvent_t *e : s->branch_events())
+    if (*e) cudaEventDestroy(*e);
   if (s->side2) cudaStreamDestroy(s->side2);
   if (s->side) cudaStreamDestroy(s->side);
   if (s->stream) cudaStreamDestroy(s->stream);

@@ -49,15 +49,19 @@ struct svof_solver {
   int ysolve_kt = 32;       // wavenumber lines per block of the DCT y solve
   // predictor Thomas coefficients, one table per substep (k_tdm_coef)
   svof::DevBuf coef;
-  // side stream of the step graph: the coefficient kernel runs beside the
-  // interface kernels
-  cudaStream_t side = nullptr;
-  // the branch of the three substeps' Thomas tables (computed at the start
-  // of a step) and its join event
-  cudaStream_t side2 = nullptr;
-  cudaEvent_t ev_coef = nullptr;
-  cudaEvent_t ev_fork[3] = {nullptr, nullptr, nullptr}, ev_join[3] = {nullptr, nullptr, nullptr};
-  cudaEvent_t ev_geom[3] = {nullptr, nullptr, nullptr};
+  // branches of a step beside the solver's stream (launch_substeps): the
+  // interface's kernels, and the three substeps' Thomas tables
+  cudaStream_t side = nullptr, side2 = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_dt = nullptr, ev_coef = nullptr;
+  cudaEvent_t ev_force[3] = {}, ev_vof[3] = {}, ev_predict[2] = {}, ev_project[2] = {};
+  std::vector<cudaEvent_t *> branch_events() {
+    std::vector<cudaEvent_t *> v{&ev_fork, &ev_dt, &ev_coef};
+    for (cudaEvent_t &e : ev_force) v.push_back(&e);
+    for (cudaEvent_t &e : ev_vof) v.push_back(&e);
+    for (cudaEvent_t &e : ev_predict) v.push_back(&e);
+    for (cudaEvent_t &e : ev_project) v.push_back(&e);
+    return v;
+  }
   // predict launch shape
   // large grids: the line-streaming predictor (k_predict_rhs, _xsolve,
   // _update) with its line array
@@ -149,9 +153,11 @@ int check_status(svof_solver *s, const char *who);
 int launch_coef(svof_solver *s, int rk, cudaStream_t st);
 // the predictor's Thomas table of substep rk (k_tdm_coef layout)
 double *coef_table(svof_solver *s, int rk);
-int launch_geom(svof_solver *s);
+int launch_geom(svof_solver *s, cudaStream_t st = nullptr);
 int launch_force(svof_solver *s, cudaStream_t st = nullptr);
-int launch_vof(svof_solver *s, int rk);
+int launch_vof(svof_solver *s, int rk, cudaStream_t st = nullptr);
+// the three substeps of a step on the solver's stream and its branches
+int launch_substeps(svof_solver *s, bool with_dt, const std::function<int(int, cudaStream_t, bool)> &tape);
 // with_coef: launch k_tdm_coef first on the same stream
 int launch_predict(svof_solver *s, int rk, bool with_coef = true);
 // (`mark`, may be empty, is called with the kernel kind after each launch)
