@@ -48,8 +48,11 @@ namespace svof3 {
 // the last row or 0 when that row is zeroed (src/tdm.c:17-50);  V[i] = v_i.
 #if SVOF3_WITH_F64
 __global__ void k3_tdm_coef(const double *__restrict__ lap_ux, const double *__restrict__ lap_cc,
-                            const double *__restrict__ dtp, double gam, double m_dif, double t_dif, int nx,
-                            double *__restrict__ coef) {
+                            const double *__restrict__ dtp, Gam3 gams, double m_dif, double t_dif, int nx,
+                            double *__restrict__ coef_all) {
+  // block b: the table of gamma = gams.g[b] at coef_all + 9 nx b
+  const double gam = gams.g[blockIdx.x];
+  double *coef = coef_all + (size_t)9 * nx * blockIdx.x;
   extern __shared__ double slap[];  // [2][3 nx]
 #pragma unroll 4
   for (int w = threadIdx.x; w < 3 * nx; w += blockDim.x) {

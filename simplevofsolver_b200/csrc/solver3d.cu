@@ -108,6 +108,19 @@ struct svof3d_solver {
   double dy = 0., dz = 0.;
   int log2ny = 0, log2nz = 0;
   cudaStream_t stream = nullptr;
+  // branches of a step beside the solver's stream (launch_substeps): the
+  // interface's kernels, and the three substeps' Thomas tables
+  cudaStream_t side = nullptr, side2 = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_dt = nullptr, ev_coef = nullptr;
+  cudaEvent_t ev_force[3] = {}, ev_vof[3] = {}, ev_predict[2] = {}, ev_project[2] = {};
+  std::vector<cudaEvent_t *> branch_events() {
+    std::vector<cudaEvent_t *> v{&ev_fork, &ev_dt, &ev_coef};
+    for (cudaEvent_t &e : ev_force) v.push_back(&e);
+    for (cudaEvent_t &e : ev_vof) v.push_back(&e);
+    for (cudaEvent_t &e : ev_predict) v.push_back(&e);
+    for (cudaEvent_t &e : ev_project) v.push_back(&e);
+    return v;
+  }
   DevBuf ux[2], uy[2], uz[2], t[2], vof[2];
   DevBuf p, psi, curv, normal, ifrcx, ifrcy, ifrcz;
   DevBuf sux[2], suy[2], suz[2], st[2], svof[2];
@@ -210,31 +223,38 @@ int launch_dt(svof3d_solver *s) {
 }
 
 template <class R>
-int launch_geom_t(svof3d_solver *s) {
-  CK(interface_geom<R>(s->stream, s->vof[s->cur_v].p, s->normal.as<R>(), s->curv.as<R>(), s->d_work, s->d_nwork,
+int launch_geom_t(svof3d_solver *s, cudaStream_t st) {
+  CK(interface_geom<R>(st, s->vof[s->cur_v].p, s->normal.as<R>(), s->curv.as<R>(), s->d_work, s->d_nwork,
                        s->grid(), s->d_health));
   return 0;
 }
-int launch_geom(svof3d_solver *s) { return s->mixed ? launch_geom_t<float>(s) : launch_geom_t<double>(s); }
+int launch_geom(svof3d_solver *s, cudaStream_t st = nullptr) {
+  if (!st) st = s->stream;
+  return s->mixed ? launch_geom_t<float>(s, st) : launch_geom_t<double>(s, st);
+}
 
 template <class R>
-int launch_force_t(svof3d_solver *s) {
-  CK(interface_force<R>(s->stream, s->vof[s->cur_v].p, s->curv.as<R>(), s->ifrcx.as<R>(), s->ifrcy.as<R>(),
+int launch_force_t(svof3d_solver *s, cudaStream_t st) {
+  CK(interface_force<R>(st, s->vof[s->cur_v].p, s->curv.as<R>(), s->ifrcx.as<R>(), s->ifrcy.as<R>(),
                         s->ifrcz.as<R>(), s->prm.tension, s->grid()));
   return 0;
 }
-int launch_force(svof3d_solver *s) { return s->mixed ? launch_force_t<float>(s) : launch_force_t<double>(s); }
+int launch_force(svof3d_solver *s, cudaStream_t st = nullptr) {
+  if (!st) st = s->stream;
+  return s->mixed ? launch_force_t<float>(s, st) : launch_force_t<double>(s, st);
+}
 
-int launch_vof(svof3d_solver *s, int rk) {
+int launch_vof(svof3d_solver *s, int rk, cudaStream_t st = nullptr) {
+  if (!st) st = s->stream;
   if (0 != rk) s->sa_v ^= 1;
   RK c{RK_A[rk], RK_B[rk], RK_A[rk] + RK_B[rk]};
   const int cv = s->cur_v, cu = s->cur_u;
   if (s->mixed) {
-    CK(interface_advect<float>(s->stream, s->vof[cv].p, s->vof[1 - cv].p, s->ux[cu].p, s->uy[cu].p, s->uz[cu].p,
+    CK(interface_advect<float>(st, s->vof[cv].p, s->vof[1 - cv].p, s->ux[cu].p, s->uy[cu].p, s->uz[cu].p,
                                s->normal.as<float>(), s->svof[s->sa_v].p, s->svof[1 - s->sa_v].p, s->d_dt, c,
                                rk != 0, s->grid()));
   } else {
-    CK(interface_advect<double>(s->stream, s->vof[cv].p, s->vof[1 - cv].p, s->ux[cu].p, s->uy[cu].p, s->uz[cu].p,
+    CK(interface_advect<double>(st, s->vof[cv].p, s->vof[1 - cv].p, s->ux[cu].p, s->uy[cu].p, s->uz[cu].p,
                                 s->normal.as<double>(), s->svof[s->sa_v].p, s->svof[1 - s->sa_v].p, s->d_dt, c,
                                 rk != 0, s->grid()));
   }
@@ -267,7 +287,7 @@ int launch_predict_t(svof3d_solver *s, int rk) {
   a.fw = s->fw.as<R>();
   a.lap_ux = s->lap_ux.p;
   a.lap_cc = s->lap_cc.p;
-  a.coef = s->coef.p;
+  a.coef = s->coef.p + (size_t)9 * s->nx * rk;
   a.dtp = s->d_dt;
   a.m_dif = s->prm.m_dif;
   a.t_dif = s->prm.t_dif;
@@ -292,11 +312,20 @@ int launch_predict_t(svof3d_solver *s, int rk) {
   return 0;
 }
 
-int launch_predict(svof3d_solver *s, int rk) {
-  k3_tdm_coef<<<1, 256, sizeof(double) * 6 * s->nx, s->stream>>>(s->lap_ux.p, s->lap_cc.p, s->d_dt,
-                                                                 RK_A[rk] + RK_B[rk], s->prm.m_dif, s->prm.t_dif,
-                                                                 s->nx, s->coef.p);
+// the predictor's Thomas tables (9 nx values a substep): of substep rk, or of
+// all three (rk < 0; they need only dt), one block each
+int launch_coef(svof3d_solver *s, int rk, cudaStream_t st) {
+  Gam3 g{};
+  for (int q = 0; q < 3; q++) g.g[q] = (rk < 0) ? RK_A[q] + RK_B[q] : RK_A[rk] + RK_B[rk];
+  k3_tdm_coef<<<rk < 0 ? 3 : 1, 256, sizeof(double) * 6 * s->nx, st>>>(
+      s->lap_ux.p, s->lap_cc.p, s->d_dt, g, s->prm.m_dif, s->prm.t_dif, s->nx,
+      s->coef.p + (size_t)9 * s->nx * std::max(rk, 0));
   CK_LAUNCH();
+  return 0;
+}
+
+int launch_predict(svof3d_solver *s, int rk, bool with_coef = true) {
+  if (with_coef && launch_coef(s, rk, s->stream)) return 1;
   if (0 != rk) s->sa_f ^= 1;
   const int rc = s->mixed ? launch_predict_t<float>(s, rk) : launch_predict_t<double>(s, rk);
   if (rc) return 1;
@@ -382,15 +411,62 @@ int launch_project(svof3d_solver *s, int rk, int do_vel, int do_p) {
   return 0;
 }
 
-int launch_step(svof3d_solver *s) {
-  if (launch_dt(s)) return 1;
-  for (int rk = 0; rk < 3; rk++) {
-    if (launch_geom(s) || launch_force(s) || launch_vof(s, rk) || launch_predict(s, rk) ||
-        launch_potential(s, rk) || launch_project(s, rk, 1, 1))
-      return 1;
+// The three substeps of a step after the time step is known (with_dt: computed
+// here).  Grids of up to kBranchCells cells run them as two branches, as the
+// 2D step does: the geometry and force of substep k + 1 and the advection of
+// substep k beside the predictor, the Poisson solve and the projection of
+// substep k (the advection waits for the previous projection, the predictor
+// for its force, and for the advected vof where that is buoyant, the next
+// force for the predictor that still reads this one's arrays).  Larger grids
+// fill the chip with each kernel and lose by it.  In line against two
+// branches: 61 x 64 x 32 four steps 1292 / 1076 us, 128^3 mixed restart stream
+// 9.12 / 8.81 ms, 256^3 step 8.40 / 8.47, 512^3 63.3 / 65.9 ms.  The three
+// substeps' predictor coefficients need dt alone and have a branch of their
+// own at every size (a launch of 8 us a substep at 256 rows).
+// tape (may be empty): called with (substep, stream, the interface's branch)
+// where the branch holds that substep's inputs
+constexpr long kBranchCells = 1L << 22;
+int launch_substeps(svof3d_solver *s, bool with_dt, const std::function<int(int, cudaStream_t, bool)> &tape) {
+  const bool branch = (long)s->nx * s->ny * s->nz <= kBranchCells;
+  cudaStream_t side = branch ? s->side : s->stream;
+  auto record = [&](cudaEvent_t e, cudaStream_t st) -> int {
+    CK(cudaEventRecord(e, st));
+    return 0;
+  };
+  auto wait = [&](cudaStream_t st, cudaEvent_t e) -> int {
+    CK(cudaStreamWaitEvent(st, e, 0));
+    return 0;
+  };
+  if (branch) {
+    if (record(s->ev_fork, s->stream) || wait(side, s->ev_fork)) return 1;
+    if (launch_geom(s, side) || launch_force(s, side) || record(s->ev_force[0], side)) return 1;
   }
-  return 0;
+  if (with_dt && launch_dt(s)) return 1;
+  if (record(s->ev_dt, s->stream) || wait(s->side2, s->ev_dt)) return 1;
+  if (launch_coef(s, -1, s->side2) || record(s->ev_coef, s->side2)) return 1;
+  if (branch && wait(side, s->ev_dt)) return 1;
+  for (int rk = 0; rk < 3; rk++) {
+    if (!branch && (launch_geom(s) || launch_force(s))) return 1;
+    if (branch && rk > 0 && wait(side, s->ev_project[rk - 1])) return 1;
+    if (tape && (tape(rk, side, true) || tape(rk, s->stream, false))) return 1;
+    if (launch_vof(s, rk, side)) return 1;
+    if (branch) {
+      if (record(s->ev_vof[rk], side) || (rk < 2 && launch_geom(s, side))) return 1;
+      if (wait(s->stream, s->ev_force[rk]) || (0. != s->grav_vof && wait(s->stream, s->ev_vof[rk]))) return 1;
+    }
+    if (0 == rk && wait(s->stream, s->ev_coef)) return 1;
+    if (launch_predict(s, rk, false)) return 1;
+    if (branch && rk < 2) {
+      if (record(s->ev_predict[rk], s->stream) || wait(side, s->ev_predict[rk])) return 1;
+      if (launch_force(s, side) || record(s->ev_force[rk + 1], side)) return 1;
+    }
+    if (launch_potential(s, rk) || launch_project(s, rk, 1, 1)) return 1;
+    if (branch && rk < 2 && record(s->ev_project[rk], s->stream)) return 1;
+  }
+  return branch ? wait(s->stream, s->ev_vof[2]) : 0;
 }
+
+int launch_step(svof3d_solver *s) { return launch_substeps(s, true, {}); }
 
 int state_key(const svof3d_solver *s) { return s->cur_u | (s->cur_v << 1) | (s->sa_f << 2) | (s->sa_v << 3); }
 
@@ -597,6 +673,10 @@ int svof3d_destroy(svof3d_solver_t *s) {
   if (s->d_work) cudaFree(s->d_work);
   if (s->d_nwork) cudaFree(s->d_nwork);
   if (s->h_dt) cudaFreeHost(s->h_dt);
+  for (cudaEvent_t *e : s->branch_events())
+    if (*e) cudaEventDestroy(*e);
+  if (s->side2) cudaStreamDestroy(s->side2);
+  if (s->side) cudaStreamDestroy(s->side);
   if (s->stream) cudaStreamDestroy(s->stream);
   delete s;
   return 0;
@@ -631,6 +711,11 @@ int svof3d_create(const svof3d_params_t *prm, const double *xf, const double *xc
     delete s;
     return fail("svof3d_create: no CUDA device available (%s)", cudaGetErrorString(cudaGetLastError()));
   }
+  if (cudaSuccess != cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking) ||
+      cudaSuccess != cudaStreamCreateWithFlags(&s->side2, cudaStreamNonBlocking))
+    return fail("svof3d_create: stream"), bail();
+  for (cudaEvent_t *e : s->branch_events())
+    if (cudaSuccess != cudaEventCreateWithFlags(e, cudaEventDisableTiming)) return fail("svof3d_create: event"), bail();
   const size_t nx = s->nx, ny = s->ny, nz = s->nz;
   const size_t es = s->mixed ? sizeof(float) : sizeof(double);  // intermediates
   const size_t n_ux = (nx + 1) * (ny + 2) * (nz + 2), n_cc = (nx + 2) * (ny + 2) * (nz + 2);
@@ -649,7 +734,7 @@ int svof3d_create(const svof3d_params_t *prm, const double *xf, const double *xc
       dalloc(s->diag, 8 + 5 * (size_t)((nx + 31) / 32) * ((ny + 7) / 8) * ((nz + kDiagPlanes - 1) / kDiagPlanes)))
     return bail();
   if (build_tables(s, xf, xc)) return bail();
-  if (dalloc(s->coef, 9 * nx)) return bail();
+  if (dalloc(s->coef, 27 * nx)) return bail();  // one table per substep
   const size_t nky = ny / 2 + 1;
   if (dalloc(s->spec, 2 * nx * nky * nz) || dalloc(s->xaux, nx * nky * nz) ||
       dalloc(s->fw, 4 * nx * ny * nz, es))
@@ -1324,15 +1409,13 @@ template <class S>
 int adj3_predict_t(svof3d_solver *s, int rk, double dt, const double *ux, const double *uy, const double *uz,
                    const double *vof_post) {
   Adjoint3State *a = s->adj;
-  k3_tdm_coef<<<1, 256, sizeof(double) * 6 * s->nx, s->stream>>>(s->lap_ux.p, s->lap_cc.p, s->d_dt,
-                                                                 RK_A[rk] + RK_B[rk], s->prm.m_dif, s->prm.t_dif,
-                                                                 s->nx, s->coef.p);
-  CK_LAUNCH();
+  if (launch_coef(s, rk, s->stream)) return 1;
   const long lines = (long)s->ny * s->nz;
   // the forward sweep's values: src_g_bar itself (FP64 intermediates) or the FP64 scratch
   double *zx = a->f32 ? a->zx.p : a->sg_x.p, *zy = a->f32 ? a->zy.p : a->sg_y.p;
   double *zz = a->f32 ? a->zz.p : a->sg_z.p;
-  CK(adj3_xsolve_launch<S>(s->stream, lines, a->xs_smem, a->ux.p, a->uy.p, a->uz.p, s->coef.p, a->sa_x.as<S>(),
+  CK(adj3_xsolve_launch<S>(s->stream, lines, a->xs_smem, a->ux.p, a->uy.p, a->uz.p,
+                            s->coef.p + (size_t)9 * s->nx * rk, a->sa_x.as<S>(),
                             a->sg_x.as<S>(), a->sa_y.as<S>(), a->sg_y.as<S>(), a->sa_z.as<S>(), a->sg_z.as<S>(),
                             a->pend_x.as<S>(), a->pend_y.as<S>(), a->pend_z.as<S>(), zx, zy, zz, RK_A[rk] * dt,
                             RK_B[rk] * dt, (RK_A[rk] + RK_B[rk]) * dt, s->grid()));
@@ -1481,20 +1564,19 @@ int svof3d_integrate_fixed(svof3d_solver_t *s, double dt, double *tape) {
   if (!(dt > 0.)) return fail("svof3d_integrate_fixed: dt must be positive");
   if (adj3_set_dt(s, dt)) return 1;
   const size_t nu = n_ux3(s), nc = n_cc3(s), nv = n_vof3(s), st = tape_stride3(s);
-  for (int rk = 0; rk < 3; rk++) {
-    if (tape) {
-      double *t = tape + rk * st;
-      const int cu = s->cur_u;
-      CK(cudaMemcpyAsync(t, s->ux[cu].p, sizeof(double) * nu, cudaMemcpyDeviceToDevice, s->stream));
-      CK(cudaMemcpyAsync(t + nu, s->uy[cu].p, sizeof(double) * nc, cudaMemcpyDeviceToDevice, s->stream));
-      CK(cudaMemcpyAsync(t + nu + nc, s->uz[cu].p, sizeof(double) * nc, cudaMemcpyDeviceToDevice, s->stream));
-      CK(cudaMemcpyAsync(t + nu + 2 * nc, s->vof[s->cur_v].p, sizeof(double) * nv, cudaMemcpyDeviceToDevice,
-                         s->stream));
+  auto record = [&](int rk, cudaStream_t stream, bool interface) -> int {
+    double *t = tape + rk * st;
+    const int cu = s->cur_u;
+    if (interface) {
+      CK(cudaMemcpyAsync(t + nu + 2 * nc, s->vof[s->cur_v].p, sizeof(double) * nv, cudaMemcpyDeviceToDevice, stream));
+    } else {
+      CK(cudaMemcpyAsync(t, s->ux[cu].p, sizeof(double) * nu, cudaMemcpyDeviceToDevice, stream));
+      CK(cudaMemcpyAsync(t + nu, s->uy[cu].p, sizeof(double) * nc, cudaMemcpyDeviceToDevice, stream));
+      CK(cudaMemcpyAsync(t + nu + nc, s->uz[cu].p, sizeof(double) * nc, cudaMemcpyDeviceToDevice, stream));
     }
-    if (launch_geom(s) || launch_force(s) || launch_vof(s, rk) || launch_predict(s, rk) ||
-        launch_potential(s, rk) || launch_project(s, rk, 1, 1))
-      return 1;
-  }
+    return 0;
+  };
+  if (tape ? launch_substeps(s, false, record) : launch_substeps(s, false, {})) return 1;
   if (tape)
     CK(cudaMemcpyAsync(tape + 3 * st, s->vof[s->cur_v].p, sizeof(double) * nv, cudaMemcpyDeviceToDevice,
                        s->stream));

@@ -145,10 +145,14 @@ template <class R>
 cudaError_t predict_launch(cudaStream_t st, const Predict3Args<R> &a);
 // opt-in shared memory of the right-hand-side kernel (once per device)
 cudaError_t predict_prepare();
-// Thomas coefficients of one substep for the three distinct systems
+// Thomas coefficients of up to three substeps for the three distinct systems,
+// one block a substep
+struct Gam3 {
+  double g[3];
+};
 __global__ void k3_tdm_coef(const double *__restrict__ lap_ux, const double *__restrict__ lap_cc,
-                            const double *__restrict__ dtp, double gam, double m_dif, double t_dif, int nx,
-                            double *__restrict__ coef);
+                            const double *__restrict__ dtp, Gam3 gams, double m_dif, double t_dif, int nx,
+                            double *__restrict__ coef_all);
 
 // Poisson: spectral array S[kz][ky][i] (complex, i fastest)
 // Poisson stages (k3_poisson.cu), templates on R, the type of the spectrum,
