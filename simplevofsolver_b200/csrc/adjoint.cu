@@ -54,7 +54,7 @@ int adj_ensure(svof_solver *s) {
              dalloc(a->pend_x, nf) || dalloc(a->pend_y, nc) || dalloc(a->sa_x, nf) || dalloc(a->sg_x, nf) ||
              dalloc(a->sa_y, nc) || dalloc(a->sg_y, nc) || dalloc(a->ifx, nf) || dalloc(a->ify, nc) ||
              dalloc(a->kap, nc) || dalloc(a->m, 2 * nc) || dalloc(a->nrm, 3 * nc) || dalloc(a->sig, nc) ||
-             dalloc(a->grv, nc) || dalloc(a->psib, nc) || dalloc(a->psis, ncc) || dalloc(a->sum, 1);
+             dalloc(a->grv, nc) || dalloc(a->psib, nc) || dalloc(a->psis, ncc) || dalloc(a->sum, 1 + kAdjSumBlocks);
   // transposed line solves: R rows per block so that the blocks cover the SMs,
   // within 160 KB of staged rows
   int r = std::max(1, std::min(8, ny / 148));
@@ -414,7 +414,9 @@ int svof_adjoint_interface_compute_curvature_tensor(svof_solver_t *s) {
 // the deterministic sum of a per-cell accumulator, copied to the host
 static int adj_total(svof_solver *s, const DevBuf &b, double *out) {
   AdjointState *a = s->adj;
-  k_adj_sum<<<1, 256, 0, s->stream>>>(b.p, (long)b.n, a->sum.p);
+  k_adj_sum<<<kAdjSumBlocks, 256, 0, s->stream>>>(b.p, (long)b.n, a->sum.p + 1);
+  CK_LAUNCH();
+  k_adj_sum<<<1, 256, 0, s->stream>>>(a->sum.p + 1, kAdjSumBlocks, a->sum.p);
   CK_LAUNCH();
   CK(cudaMemcpyAsync(out, a->sum.p, sizeof(double), cudaMemcpyDeviceToHost, s->stream));
   CK(cudaStreamSynchronize(s->stream));

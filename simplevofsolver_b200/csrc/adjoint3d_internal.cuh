@@ -96,6 +96,7 @@ cudaError_t adj3_corners_launch(cudaStream_t st, const double *vof, const S *am,
                                 double *avof, AGrid3 ag);
 
 // deterministic sum (one block of 256 threads)
+constexpr int kAdjSumBlocks = 592;
 __global__ void k3_adj_sum(const double *__restrict__ x, long n, double *__restrict__ out);
 // *dst = v in stream order
 __global__ void k3_adj_set(double *dst, double v);

@@ -54,6 +54,7 @@ constexpr int CBX = 32, CBY = 8;
 __global__ void k_adj_corners(const double *__restrict__ vof, const double *__restrict__ am,
                               const double *__restrict__ akap, double *__restrict__ avof, Grid2 g);
 // deterministic sum (one block of 256 threads)
+constexpr int kAdjSumBlocks = 592;
 __global__ void k_adj_sum(const double *__restrict__ x, long n, double *__restrict__ out);
 // *dst = v in stream order
 __global__ void k_adj_set(double *dst, double v);

@@ -773,18 +773,20 @@ __global__ void k3_adj_cvof(const S *__restrict__ gbar, double *__restrict__ avo
   avof[ix_src(g, i, j, k)] += sx + sy * ag.rdy + sz * ag.rdz;
 }
 
-// deterministic sum of n values (one block of 256 threads)
+// deterministic sum of n values: block b's share into out[b] (a thread's
+// values in order, the threads by a fixed tree); the callers sum kAdjSumBlocks
+// shares in a second launch (one block alone took 1.2 ms at 128^3)
 __global__ void k3_adj_sum(const double *__restrict__ x, long n, double *__restrict__ out) {
   __shared__ double part[256];
   double s = 0.;
-  for (long q = threadIdx.x; q < n; q += blockDim.x) s += x[q];
+  for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long)gridDim.x * blockDim.x) s += x[q];
   part[threadIdx.x] = s;
   __syncthreads();
   for (int w = blockDim.x / 2; w > 0; w >>= 1) {
     if ((int)threadIdx.x < w) part[threadIdx.x] += part[threadIdx.x + w];
     __syncthreads();
   }
-  if (0 == threadIdx.x) *out = part[0];
+  if (0 == threadIdx.x) out[blockIdx.x] = part[0];
 }
 
 __global__ void k3_adj_set(double *dst, double v) { *dst = v; }

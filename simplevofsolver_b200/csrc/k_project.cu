@@ -180,8 +180,12 @@ __global__ void k_dt_final(unsigned long long *minbits, double *dt, double coef_
 }
 
 // ---------------------------------------------------------------------------
-// k_diag: one block, deterministic order; out = {divmax, vofmin, vofmax,
-// sum vof dx dy, sum dx dy}.  Sums use a TwoSum-compensated accumulation.
+// Two deterministic stages each for k_diag and k_logging: reduce_blocks(n)
+// blocks of kRedThreads threads write their partials, one block folds them in
+// a fixed order.  Sums are TwoSum-compensated: a thread's terms, a warp's
+// partials by a fixed butterfly, the warps and blocks in order.  (One block of
+// 1024 threads over the whole grid before: 90 and 145 us at 128 x 256, now 5
+// and 8 with the fold.)
 __device__ __forceinline__ void two_sum_acc(double &s, double &c, double x) {
   const double t = s + x;
   const double bp = t - s;
@@ -190,59 +194,7 @@ __device__ __forceinline__ void two_sum_acc(double &s, double &c, double x) {
   c += err;
 }
 
-__global__ void k_diag(const double *__restrict__ ux, const double *__restrict__ uy,
-                       const double *__restrict__ vof, double *__restrict__ out, Grid2 g) {
-  const int nx = g.nx, ny = g.ny;
-  double dmax = 0., vmin = 1., vmax = 0., s0 = 0., c0 = 0., s1 = 0., c1 = 0.;
-  for (long w = threadIdx.x; w < (long)nx * ny; w += blockDim.x) {
-    const int i = 1 + (int)(w % nx), j = 1 + (int)(w / nx);
-    const double dx = g.dxf[i - 1];
-    const double div = +(ux[ix_ux(nx, i + 1, j)] - ux[ix_ux(nx, i, j)]) / dx +
-                       (uy[ix_cc(nx, i, j + 1)] - uy[ix_cc(nx, i, j)]) / g.dy;
-    dmax = fmax(dmax, fabs(div));
-    const double lv = vof[ix_vof(nx, i, j)];
-    vmin = fmin(vmin, lv);
-    vmax = fmax(vmax, lv);
-    two_sum_acc(s0, c0, lv * (dx * g.dy));
-    two_sum_acc(s1, c1, dx * g.dy);
-  }
-  __shared__ double red[5][1024];
-  red[0][threadIdx.x] = dmax;
-  red[1][threadIdx.x] = vmin;
-  red[2][threadIdx.x] = vmax;
-  red[3][threadIdx.x] = s0 + c0;
-  red[4][threadIdx.x] = s1 + c1;
-  __syncthreads();
-  if (0 == threadIdx.x) {
-    double a = 0., b = 1., c = 0., ss0 = 0., cc0 = 0., ss1 = 0., cc1 = 0.;
-    for (int t = 0; t < (int)blockDim.x; t++) {
-      a = fmax(a, red[0][t]);
-      b = fmin(b, red[1][t]);
-      c = fmax(c, red[2][t]);
-      two_sum_acc(ss0, cc0, red[3][t]);
-      two_sum_acc(ss1, cc1, red[4][t]);
-    }
-    out[0] = a;
-    out[1] = b;
-    out[2] = c;
-    out[3] = ss0 + cc0;
-    out[4] = ss1 + cc1;
-  }
-}
-
-// ---------------------------------------------------------------------------
-// k_logging: the logging reductions of src/logging/momentum.c:38-54,
-// energy.c:41-65 and nusselt/{heat_flux,kinetic_energy_injection,
-// kinetic_energy_dissipation,thermal_energy_dissipation}.c on the device,
-// every term with the reference's expression and association; the sums are
-// TwoSum-compensated, thread partials folded over a warp by a fixed
-// butterfly and over the block in warp order (deterministic).  One block of
-// kLogThreads threads walks the positions (i, j), i in [1, nx+1], j in
-// [1, ny].  out = {momentum x, y; energy ux, uy, t; Nusselt from the wall
-// heat flux, kinetic energy injection, kinetic and thermal energy
-// dissipation}.
 namespace {
-constexpr int kLogThreads = 1024, kLogSums = 13;
 struct CSum {
   double s = 0., c = 0.;
   __device__ __forceinline__ void add(double x) { two_sum_acc(s, c, x); }
@@ -250,12 +202,119 @@ struct CSum {
     two_sum_acc(s, c, o.s);
     c += o.c;
   }
+  // over the warp, in a fixed order
+  __device__ __forceinline__ void warp() {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      CSum x;
+      x.s = __shfl_xor_sync(0xffffffffu, s, o);
+      x.c = __shfl_xor_sync(0xffffffffu, c, o);
+      add(x);
+    }
+  }
 };
+
+// the block's NS sums into part[2 q], part[2 q + 1] of this block
+template <int NS>
+__device__ __forceinline__ void block_sums(CSum *sum, double *__restrict__ part) {
+  __shared__ CSum red[NS][kRedThreads / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int q = 0; q < NS; q++) {
+    sum[q].warp();
+    if (0 == lane) red[q][warp] = sum[q];
+  }
+  __syncthreads();
+  if (threadIdx.x < NS) {
+    const int q = threadIdx.x;
+    CSum r = red[q][0];
+    for (int w = 1; w < kRedThreads / 32; w++) r.add(red[q][w]);
+    part[2 * q] = r.s;
+    part[2 * q + 1] = r.c;
+  }
+}
+
+// sum q of the blocks' partials (stride values a block), by one warp
+__device__ __forceinline__ double fold_sum(const double *__restrict__ part, int blocks, int stride, int q) {
+  CSum r;
+  for (int b = threadIdx.x & 31; b < blocks; b += 32) {
+    CSum x;
+    x.s = part[(size_t)b * stride + 2 * q];
+    x.c = part[(size_t)b * stride + 2 * q + 1];
+    r.add(x);
+  }
+  r.warp();
+  return r.s + r.c;
+}
+__device__ __forceinline__ double warp_max(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
 }  // namespace
 
-__global__ void __launch_bounds__(kLogThreads) k_logging(const double *__restrict__ ux, const double *__restrict__ uy,
+// partials of k_diag: vof sums (vof dx dy, dx dy), then max |div u|, - vof min
+// and vof max
+__global__ void __launch_bounds__(kRedThreads) k_diag(const double *__restrict__ ux, const double *__restrict__ uy,
+                                                      const double *__restrict__ vof, double *__restrict__ part,
+                                                      Grid2 g) {
+  const int nx = g.nx, ny = g.ny;
+  double m[3] = {0., -1., 0.};
+  CSum sum[2];
+  for (long w = (long)blockIdx.x * kRedThreads + threadIdx.x; w < (long)nx * ny; w += (long)gridDim.x * kRedThreads) {
+    const int i = 1 + (int)(w % nx), j = 1 + (int)(w / nx);
+    const double dx = g.dxf[i - 1];
+    const double div = +(ux[ix_ux(nx, i + 1, j)] - ux[ix_ux(nx, i, j)]) / dx +
+                       (uy[ix_cc(nx, i, j + 1)] - uy[ix_cc(nx, i, j)]) / g.dy;
+    m[0] = fmax(m[0], fabs(div));
+    const double lv = vof[ix_vof(nx, i, j)];
+    m[1] = fmax(m[1], -lv);
+    m[2] = fmax(m[2], lv);
+    sum[0].add(lv * (dx * g.dy));
+    sum[1].add(dx * g.dy);
+  }
+  part += (size_t)kDiagPartials * blockIdx.x;
+  block_sums<2>(sum, part);
+  __shared__ double red[3][kRedThreads / 32];
+#pragma unroll
+  for (int q = 0; q < 3; q++) {
+    m[q] = warp_max(m[q]);
+    if (0 == (threadIdx.x & 31)) red[q][threadIdx.x >> 5] = m[q];
+  }
+  __syncthreads();
+  if (threadIdx.x < 3) {
+    double v = red[threadIdx.x][0];
+    for (int w = 1; w < kRedThreads / 32; w++) v = fmax(v, red[threadIdx.x][w]);
+    part[4 + threadIdx.x] = v;
+  }
+}
+
+// out = {max |div u|, vof min, vof max, sum vof dx dy, sum dx dy}
+__global__ void __launch_bounds__(5 * 32) k_diag_fold(const double *__restrict__ part, int blocks,
+                                                      double *__restrict__ out) {
+  const int q = threadIdx.x >> 5;
+  double v;
+  if (q < 3) {
+    v = 1 == q ? -1. : 0.;
+    for (int b = threadIdx.x & 31; b < blocks; b += 32) v = fmax(v, part[(size_t)b * kDiagPartials + 4 + q]);
+    v = warp_max(v);
+    if (1 == q) v = -v;
+  } else {
+    v = fold_sum(part, blocks, kDiagPartials, q - 3);
+  }
+  if (0 == (threadIdx.x & 31)) out[q] = v;
+}
+
+// ---------------------------------------------------------------------------
+// k_logging: the logging reductions of src/logging/momentum.c:38-54,
+// energy.c:41-65 and nusselt/{heat_flux,kinetic_energy_injection,
+// kinetic_energy_dissipation,thermal_energy_dissipation}.c on the device,
+// every term with the reference's expression and association, over the
+// positions (i, j), i in [1, nx+1], j in [1, ny].  Partials: kLogSums sums a
+// block.
+__global__ void __launch_bounds__(kRedThreads) k_logging(const double *__restrict__ ux, const double *__restrict__ uy,
                                                          const double *__restrict__ t, double m_dif, double t_dif,
-                                                         double ly, double *__restrict__ out, Grid2 g) {
+                                                         double *__restrict__ part, Grid2 g) {
   const int nx = g.nx, ny = g.ny;
   const double dy = g.dy, md = m_dif, td = t_dif;
   auto UX = [&](int i, int j) { return ux[ix_ux(nx, i, j)]; };
@@ -267,7 +326,7 @@ __global__ void __launch_bounds__(kLogThreads) k_logging(const double *__restric
   // dissipation (ux-x, ux-y, uy-x, uy-y), 11..12 thermal dissipation (x, y)
   CSum sum[kLogSums];
   const int npos = (nx + 1) * ny;
-  for (int w = threadIdx.x; w < npos; w += kLogThreads) {
+  for (int w = blockIdx.x * kRedThreads + threadIdx.x; w < npos; w += gridDim.x * kRedThreads) {
     const int i = 1 + w % (nx + 1), j = 1 + w / (nx + 1);
     // ---- ux faces i in [1, nx+1]
     {
@@ -338,44 +397,24 @@ __global__ void __launch_bounds__(kLogThreads) k_logging(const double *__restric
       sum[5].add(-(0.5 * td * (dtdx_xm + dtdx_xp) * dy));
     }
   }
-  // warp butterfly, then warp order
-#pragma unroll
-  for (int q = 0; q < kLogSums; q++) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      CSum x;
-      x.s = __shfl_xor_sync(0xffffffffu, sum[q].s, o);
-      x.c = __shfl_xor_sync(0xffffffffu, sum[q].c, o);
-      sum[q].add(x);
-    }
-  }
-  __shared__ CSum red[kLogSums][kLogThreads / 32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (0 == lane) {
-#pragma unroll
-    for (int q = 0; q < kLogSums; q++) red[q][warp] = sum[q];
-  }
+  block_sums<kLogSums>(sum, part + (size_t)2 * kLogSums * blockIdx.x);
+}
+
+// out = {momentum x, y; energy ux, uy, t; Nusselt from the wall heat flux,
+// kinetic energy injection, kinetic and thermal energy dissipation}
+__global__ void __launch_bounds__(kLogSums * 32) k_logging_fold(const double *__restrict__ part, int blocks,
+                                                                double t_dif, double ly, double *__restrict__ out) {
+  __shared__ double v[kLogSums];
+  const double r = fold_sum(part, blocks, 2 * kLogSums, threadIdx.x >> 5);
+  if (0 == (threadIdx.x & 31)) v[threadIdx.x >> 5] = r;
   __syncthreads();
-  if (threadIdx.x < kLogSums) {
-    const int q = threadIdx.x;
-    CSum r = red[q][0];
-    for (int w = 1; w < kLogThreads / 32; w++) r.add(red[q][w]);
-    red[q][0] = r;
-  }
-  __syncthreads();
-  if (0 == threadIdx.x) {
-    auto v = [&](int q) { return red[q][0].s + red[q][0].c; };
-    const double ref = td * ly;  // laminar heat flux (nusselt/reference.c:4-12)
-    out[0] = v(0);
-    out[1] = v(1);
-    out[2] = v(2);
-    out[3] = v(3);
-    out[4] = v(4);
-    out[5] = v(5) / ref;
-    out[6] = v(6) / ref + 1.;
-    out[7] = (((v(7) + v(8)) + v(9)) + v(10)) / ref + 1.;
-    out[8] = (v(11) + v(12)) / ref;
-  }
+  if (0 != threadIdx.x) return;
+  const double ref = t_dif * ly;  // laminar heat flux (nusselt/reference.c:4-12)
+  for (int q = 0; q < 5; q++) out[q] = v[q];
+  out[5] = v[5] / ref;
+  out[6] = v[6] / ref + 1.;
+  out[7] = (((v[7] + v[8]) + v[9]) + v[10]) / ref + 1.;
+  out[8] = (v[11] + v[12]) / ref;
 }
 
 }  // namespace svof

@@ -590,7 +590,7 @@ int engine_create(const svof_params_t *prm, const double *xf, const double *xc, 
   }
   if (dalloc(s->p, n_cc, mg) || dalloc(s->psi, n_cc, mg) || dalloc(s->curv, n_cc, mg) ||
       dalloc(s->normal, 3 * (size_t)nx * (ny + 2), mg) || dalloc(s->ifrcx, n_srcx, mg) ||
-      dalloc(s->ifrcy, n_src, mg) || dalloc(s->diag, 16))
+      dalloc(s->ifrcy, n_src, mg) || dalloc(s->diag, 16 + 2 * (size_t)kLogSums * kRedBlocks))
     return bail();
   if (build_tables(s, xf, xc)) return bail();
   if (dalloc(s->coef, 27 * (size_t)nx)) return bail();  // one table per substep
@@ -988,8 +988,11 @@ int svof_profile_step(svof_solver_t *s, double *ms, int *launches, int nkinds) {
 int svof_diagnostics(svof_solver_t *s, double *divmax, double *vofmin, double *vofmax, double *vofmean) {
   SVOF_RANGE();
   if (!s) return fail("null argument");
-  k_diag<<<1, 1024, 0, s->stream>>>(s->ux[s->cur_u].p, s->uy[s->cur_u].p, s->vof[s->cur_v].p, s->diag.p,
-                                    s->grid());
+  const int blocks = reduce_blocks((long)s->nx * s->ny);
+  k_diag<<<blocks, kRedThreads, 0, s->stream>>>(s->ux[s->cur_u].p, s->uy[s->cur_u].p, s->vof[s->cur_v].p,
+                                                s->diag.p + 16, s->grid());
+  CK_LAUNCH();
+  k_diag_fold<<<1, 5 * 32, 0, s->stream>>>(s->diag.p + 16, blocks, s->diag.p);
   CK_LAUNCH();
   double h[5];
   CK(cudaMemcpyAsync(h, s->diag.p, sizeof(h), cudaMemcpyDeviceToHost, s->stream));
@@ -1003,8 +1006,11 @@ int svof_diagnostics(svof_solver_t *s, double *divmax, double *vofmin, double *v
 
 int svof_logging_quantities(svof_solver_t *s, double *out, int nout) {
   if (!s || !out || nout < 9) return fail("svof_logging_quantities: bad arguments (nout must be >= 9)");
-  k_logging<<<1, 1024, 0, s->stream>>>(s->ux[s->cur_u].p, s->uy[s->cur_u].p, s->t[s->cur_u].p, s->prm.m_dif,
-                                       s->prm.t_dif, s->prm.ly, s->diag.p, s->grid());
+  const int blocks = reduce_blocks((long)(s->nx + 1) * s->ny);
+  k_logging<<<blocks, kRedThreads, 0, s->stream>>>(s->ux[s->cur_u].p, s->uy[s->cur_u].p, s->t[s->cur_u].p,
+                                                   s->prm.m_dif, s->prm.t_dif, s->diag.p + 16, s->grid());
+  CK_LAUNCH();
+  k_logging_fold<<<1, kLogSums * 32, 0, s->stream>>>(s->diag.p + 16, blocks, s->prm.t_dif, s->prm.ly, s->diag.p);
   CK_LAUNCH();
   CK(cudaMemcpyAsync(out, s->diag.p, 9 * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
   CK(cudaStreamSynchronize(s->stream));

@@ -1314,7 +1314,7 @@ int adj3_ensure(svof3d_solver *s) {
              dalloc(a->sg_z, nc, es) || dalloc(a->ifx, nf, es) || dalloc(a->ify, nc, es) || dalloc(a->ifz, nc, es) ||
              dalloc(a->kap, nc, es) || dalloc(a->m, 3 * nc, es) || dalloc(a->nrm, 4 * nc, es) ||
              dalloc(a->sig, nc) || dalloc(a->psib, nc) || dalloc(a->b, nc) || dalloc(a->psis, ncc) ||
-             dalloc(a->gbar, 3 * (nx + 1) * ny * nz, es) || dalloc(a->grv, nc) || dalloc(a->sum, 1);
+             dalloc(a->gbar, 3 * (nx + 1) * ny * nz, es) || dalloc(a->grv, nc) || dalloc(a->sum, 1 + kAdjSumBlocks);
   if (!bad && a->f32) bad = dalloc(a->zx, nf) || dalloc(a->zy, nc) || dalloc(a->zz, nc);
   if (!bad && s->mixed)
     bad = dalloc(a->nrm64, 4 * nx * (ny + 2) * (nz + 2)) || dalloc(a->curv64, ncc) ||
@@ -1720,7 +1720,9 @@ int svof3d_adjoint_interface_compute_curvature_tensor(svof3d_solver_t *s) {
 // the deterministic sum of a per-cell accumulator, copied to the host
 static int adj3_total(svof3d_solver *s, const DevBuf &b, double *out) {
   Adjoint3State *a = s->adj;
-  k3_adj_sum<<<1, 256, 0, s->stream>>>(b.p, (long)b.n, a->sum.p);
+  k3_adj_sum<<<kAdjSumBlocks, 256, 0, s->stream>>>(b.p, (long)b.n, a->sum.p + 1);
+  CK_LAUNCH();
+  k3_adj_sum<<<1, 256, 0, s->stream>>>(a->sum.p + 1, kAdjSumBlocks, a->sum.p);
   CK_LAUNCH();
   CK(cudaMemcpyAsync(out, a->sum.p, sizeof(double), cudaMemcpyDeviceToHost, s->stream));
   CK(cudaStreamSynchronize(s->stream));

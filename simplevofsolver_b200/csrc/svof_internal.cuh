@@ -182,13 +182,22 @@ __global__ void k_cfl(const double *__restrict__ ux, const double *__restrict__ 
                       unsigned long long *__restrict__ minbits, unsigned *__restrict__ status, Grid2 g);
 __global__ void k_dt_final(unsigned long long *minbits, double *dt, double coef_adv, double dif_m_y,
                            double dif_t_y, unsigned *status);
-// diagnostics (src/logging/divergence.c, src/logging/interface.c)
-__global__ void k_diag(const double *__restrict__ ux, const double *__restrict__ uy,
-                       const double *__restrict__ vof, double *__restrict__ out, Grid2 g);
-// logging reductions (src/logging/momentum.c, energy.c, nusselt/); one block
+// diagnostics (src/logging/divergence.c, src/logging/interface.c) and logging
+// reductions (src/logging/momentum.c, energy.c, nusselt/): partials of
+// reduce_blocks(n) blocks of kRedThreads threads, folded by one block
+constexpr int kRedThreads = 256, kRedBlocks = 296, kDiagPartials = 7, kLogSums = 13;
+inline int reduce_blocks(long n) {
+  const long b = (n + kRedThreads - 1) / kRedThreads;
+  return (int)(b < kRedBlocks ? b : kRedBlocks);
+}
+__global__ void k_diag(const double *__restrict__ ux, const double *__restrict__ uy, const double *__restrict__ vof,
+                       double *__restrict__ part, Grid2 g);
+__global__ void k_diag_fold(const double *__restrict__ part, int blocks, double *__restrict__ out);
 __global__ void k_logging(const double *__restrict__ ux, const double *__restrict__ uy,
-                          const double *__restrict__ t, double m_dif, double t_dif, double ly,
-                          double *__restrict__ out, Grid2 g);
+                          const double *__restrict__ t, double m_dif, double t_dif, double *__restrict__ part,
+                          Grid2 g);
+__global__ void k_logging_fold(const double *__restrict__ part, int blocks, double t_dif, double ly,
+                               double *__restrict__ out);
 
 // ---- engine internals shared by the C ABI front-ends (solver.cu, dropin.cu) ----
 // svof_create with a choice of field memory: managed = CUDA managed memory,
