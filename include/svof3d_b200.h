@@ -135,6 +135,9 @@ int svof3d_device_field(svof3d_solver_t *s, int field, double **dptr);
  * nz x ny x (nx+1) for ux and nz x ny x (nx+2) for uy, uz, p, t, psi, vof;
  * loading applies the field's halo and wall update */
 int svof3d_load_interior(svof3d_solver_t *s, int field, const double *host, size_t count);
+/* the same from device memory (complete on return; the caller's writes of it
+ * must be complete before the call) */
+int svof3d_load_interior_device(svof3d_solver_t *s, int field, const double *device, size_t count);
 int svof3d_store_interior(svof3d_solver_t *s, int field, double *host, size_t count);
 
 /* Queued forms of the two calls above, for streaming restart states through

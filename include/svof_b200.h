@@ -110,6 +110,9 @@ int svof_device_field(svof_solver_t *solver, int field, double **device_ptr);
  * boundaries_vof do in fluid_init (src/fluid/init.c:82-88) and
  * interface_init (src/interface/init.c:60-63). */
 int svof_load_interior(svof_solver_t *solver, int field, const double *host, size_t count);
+/* the same from device memory (complete on return; the caller's writes of it
+ * must be complete before the call) */
+int svof_load_interior_device(svof_solver_t *solver, int field, const double *device, size_t count);
 /* copies rows 1..ny of ux, uy, p, t or vof to host memory (the part
  * fluid_save / interface_save write, src/fluid/save.c:18-25) */
 int svof_store_interior(svof_solver_t *solver, int field, double *host, size_t count);

@@ -49,7 +49,7 @@ FIELDS = {"ux": 0, "uy": 1, "p": 2, "psi": 3, "t": 4, "vof": 5, "curv": 6, "norm
 
 # public C-ABI symbols (include/svof_b200.h)
 EXPORTS = ["svof_create", "svof_destroy", "svof_field_count", "svof_upload_field",
-           "svof_download_field", "svof_device_field", "svof_load_interior", "svof_store_interior",
+           "svof_download_field", "svof_device_field", "svof_load_interior", "svof_load_interior_device", "svof_store_interior",
            "svof_x_grid_is_uniform", "svof_fluid_decide_dt", "svof_interface_compute_curvature_tensor",
            "svof_interface_compute_force", "svof_interface_update_vof", "svof_fluid_predict_field",
            "svof_fluid_compute_potential_dct", "svof_fluid_compute_potential_dft",
@@ -131,6 +131,7 @@ def lib() -> ctypes.CDLL:
         L.svof_download_field.argtypes = [vp, i, dp, sz]
         L.svof_device_field.argtypes = [vp, i, ctypes.POINTER(vp)]
         L.svof_load_interior.argtypes = [vp, i, dp, sz]
+        L.svof_load_interior_device.argtypes = [vp, i, dp, sz]
         L.svof_store_interior.argtypes = [vp, i, dp, sz]
         L.svof_x_grid_is_uniform.argtypes = [vp, ctypes.POINTER(i)]
         L.svof_fluid_decide_dt.argtypes = [vp, pd]
@@ -277,6 +278,17 @@ class Solver:
         if a.shape != interior_shape(name, self.nx, self.ny):
             raise ValueError(f"{name}: expected shape {interior_shape(name, self.nx, self.ny)}, got {a.shape}")
         _check(lib().svof_load_interior(self._h, FIELDS[name], a.ctypes.data, a.size))
+
+    def load_interior_device(self, name: str, a):
+        """load_interior from a contiguous float64 CUDA tensor of the field's
+        restart shape (work on torch's current stream is waited for)"""
+        import torch
+        want = interior_shape(name, self.nx, self.ny)
+        if (not isinstance(a, torch.Tensor) or not a.is_cuda or a.dtype != torch.float64 or tuple(a.shape) != want
+                or not a.is_contiguous()):
+            raise ValueError(f"{name}: expected a contiguous float64 CUDA tensor of shape {want}")
+        torch.cuda.current_stream(a.device).synchronize()
+        _check(lib().svof_load_interior_device(self._h, FIELDS[name], a.data_ptr(), a.numel()))
 
     def interior(self, name: str) -> np.ndarray:
         out = np.empty(interior_shape(name, self.nx, self.ny))

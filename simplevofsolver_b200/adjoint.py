@@ -35,18 +35,33 @@ from __future__ import annotations
 
 import numpy as np
 
-from . import Solver, SvofError
+from . import Solver, SvofError, interior_shape, interior_shape3d
 
 
-def _to_interior(name, a, nx, ny):
-    """compact (device tensor) -> restart-file layout (numpy)"""
-    a = a.detach().to("cpu").double().numpy()
-    out = np.zeros((ny, nx + 1) if name == "ux" else (ny, nx + 2))
-    if name == "ux":
-        out[:, 1:nx] = a
-    else:
-        out[:, 1:nx + 1] = a
+def _interior(a, shape):
+    """compact (tensor) -> restart layout of the given shape on the GPU, the
+    walls zero"""
+    import torch
+    out = torch.zeros(shape, dtype=torch.float64, device="cuda")
+    out[..., 1:-1].copy_(a.detach())
     return out
+
+
+class _Held:
+    """The initial p and t of every rollout, held on the GPU: read back as
+    (read-only) arrays in the restart layout, replaced by assignment."""
+
+    def __set_name__(self, owner, name):
+        self.key = "_dev_" + name
+
+    def __get__(self, r, owner=None):
+        a = getattr(r, self.key).cpu().numpy()
+        a.flags.writeable = False
+        return a
+
+    def __set__(self, r, a):
+        import torch
+        setattr(r, self.key, torch.from_numpy(np.array(a, dtype=np.float64)).to("cuda"))
 
 
 class Rollout:
@@ -57,6 +72,7 @@ class Rollout:
     ``checkpoint_every`` = K."""
 
     STATE = ("ux", "uy", "p", "t", "vof")
+    p0, t0 = _Held(), _Held()
 
     def __init__(self, solver: Solver, dts, checkpoint_every: int = 20, project_initial: bool = True):
         import torch
@@ -83,11 +99,10 @@ class Rollout:
         s.set_tension(float(tension))
         if grav is not None:
             s.set_gravity(float(grav), s.gravity[1])
-        s.load_interior("ux", _to_interior("ux", ux0, self.nx, self.ny))
-        s.load_interior("uy", _to_interior("uy", uy0, self.nx, self.ny))
-        s.load_interior("vof", _to_interior("vof", vof0, self.nx, self.ny))
-        s.load_interior("p", self.p0)
-        s.load_interior("t", self.t0)
+        for name, a in (("ux", ux0), ("uy", uy0), ("vof", vof0)):
+            s.load_interior_device(name, _interior(a, interior_shape(name, self.nx, self.ny)))
+        s.load_interior_device("p", self._dev_p0)
+        s.load_interior_device("t", self._dev_t0)
         if self.project:
             # the discrete projection u - grad L^-1 div u of the initial
             # velocity (the Poisson solve and correction of a substep; the
@@ -207,18 +222,6 @@ def rollout(ux0, uy0, vof0, tension, r: Rollout, grav=None):
     return _RF.apply(ux0, uy0, vof0, tension, grav, r)
 
 
-def _to_interior3(name, a, nx):
-    """compact (device tensor, (nz, ny, nx-1 | nx)) -> restart interior (numpy)"""
-    a = a.detach().to("cpu").double().numpy()
-    nz, ny = a.shape[:2]
-    out = np.zeros((nz, ny, nx + 1) if name == "ux" else (nz, ny, nx + 2))
-    if name == "ux":
-        out[..., 1:nx] = a
-    else:
-        out[..., 1:nx + 1] = a
-    return out
-
-
 class Rollout3D:
     """The 3D form of :class:`Rollout`: ``len(dts)`` steps of a
     :class:`simplevofsolver_b200.solver3d.Solver3D` (precision "fp64") with
@@ -233,6 +236,7 @@ class Rollout3D:
     nx-1), cells (nz, ny, nx)."""
 
     STATE = ("ux", "uy", "uz", "p", "t", "vof")
+    p0, t0 = _Held(), _Held()
 
     def __init__(self, solver, dts, checkpoint_every: int = 20, project_initial: bool = True):
         import torch
@@ -259,9 +263,11 @@ class Rollout3D:
         if grav is not None:
             s.set_gravity(float(grav), s.gravity[1])
         for name, a in (("ux", ux0), ("uy", uy0), ("uz", uz0), ("vof", vof0)):
-            s.load_interior(name, _to_interior3(name, a, self.nx))
-        s.load_interior("p", self.p0)
-        s.load_interior("t", self.t0)
+            if tuple(a.shape[:2]) != (self.nz, self.ny):
+                raise ValueError(f"{name}: expected {self.nz} planes of {self.ny} rows, got {tuple(a.shape)}")
+            s.load_interior_device(name, _interior(a, interior_shape3d(name, self.nx, self.ny, self.nz)))
+        s.load_interior_device("p", self._dev_p0)
+        s.load_interior_device("t", self._dev_t0)
         if self.project:
             s.fluid_compute_potential_dft(0, 1.0)
             s.fluid_correct_velocity(0, 1.0)

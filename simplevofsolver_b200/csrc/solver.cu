@@ -775,18 +775,27 @@ int svof_device_field(svof_solver_t *s, int field, double **dptr) {
   return 0;
 }
 
-int svof_load_interior(svof_solver_t *s, int field, const double *host, size_t count) {
-  SVOF_RANGE();
+static int load_interior(svof_solver_t *s, int field, const double *src, size_t count, cudaMemcpyKind kind) {
   int nh, width;
   DevBuf *b;
-  if (!s || !host) return fail("null argument");
+  if (!s || !src) return fail("null argument");
   if (interior_layout(s, field, &nh, &width) || field_buf(s, field, &b)) return 1;
   const size_t n = (size_t)width * s->ny;
   if (count != n) return fail("field %d: restart layout holds %zu doubles, got %zu", field, n, count);
-  CK(cudaMemcpyAsync(b->p + (size_t)nh * width, host, sizeof(double) * n, cudaMemcpyHostToDevice, s->stream));
+  CK(cudaMemcpyAsync(b->p + (size_t)nh * width, src, sizeof(double) * n, kind, s->stream));
   if (launch_halo_bc(s, b->p, field)) return 1;
   CK(cudaStreamSynchronize(s->stream));
   return 0;
+}
+
+int svof_load_interior(svof_solver_t *s, int field, const double *host, size_t count) {
+  SVOF_RANGE();
+  return load_interior(s, field, host, count, cudaMemcpyHostToDevice);
+}
+
+int svof_load_interior_device(svof_solver_t *s, int field, const double *device, size_t count) {
+  SVOF_RANGE();
+  return load_interior(s, field, device, count, cudaMemcpyDeviceToDevice);
 }
 
 int svof_store_interior(svof_solver_t *s, int field, double *host, size_t count) {

@@ -829,11 +829,10 @@ int svof3d_device_field(svof3d_solver_t *s, int field, double **dptr) {
 
 // the restart layout is nz x ny x width; in storage each interior plane k has
 // nh halo rows below and above, so the copy is one 2D memcpy of nz planes
-int svof3d_load_interior(svof3d_solver_t *s, int field, const double *host, size_t count) {
-  SVOF_RANGE();
+static int load_interior(svof3d_solver_t *s, int field, const double *src, size_t count, cudaMemcpyKind kind) {
   int nh, width;
   DevBuf *b;
-  if (!s || !host) return fail("null argument");
+  if (!s || !src) return fail("null argument");
   if (interior_layout(s, field, &nh, &width) || field_buf(s, field, &b)) return 1;
   const size_t plane = (size_t)width * s->ny;
   if (count != plane * s->nz) return fail("field %d: restart layout holds %zu doubles, got %zu", field,
@@ -841,10 +840,20 @@ int svof3d_load_interior(svof3d_solver_t *s, int field, const double *host, size
   const size_t spitch = sizeof(double) * plane;
   const size_t dpitch = sizeof(double) * (size_t)width * (s->ny + 2 * nh);
   double *dst = b->p + (size_t)width * (s->ny + 2 * nh) * nh + (size_t)width * nh;
-  CK(cudaMemcpy2DAsync(dst, dpitch, host, spitch, spitch, s->nz, cudaMemcpyHostToDevice, s->stream));
+  CK(cudaMemcpy2DAsync(dst, dpitch, src, spitch, spitch, s->nz, kind, s->stream));
   if (launch_halo_bc(s, b->p, field)) return 1;
   CK(cudaStreamSynchronize(s->stream));
   return 0;
+}
+
+int svof3d_load_interior(svof3d_solver_t *s, int field, const double *host, size_t count) {
+  SVOF_RANGE();
+  return load_interior(s, field, host, count, cudaMemcpyHostToDevice);
+}
+
+int svof3d_load_interior_device(svof3d_solver_t *s, int field, const double *device, size_t count) {
+  SVOF_RANGE();
+  return load_interior(s, field, device, count, cudaMemcpyDeviceToDevice);
 }
 
 int svof3d_store_interior(svof3d_solver_t *s, int field, double *host, size_t count) {

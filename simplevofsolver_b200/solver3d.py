@@ -38,7 +38,8 @@ FIELDS3D = {"ux": 0, "uy": 1, "uz": 2, "p": 3, "t": 4, "vof": 5, "psi": 6, "curv
             "srcuz_a": 16, "srcuz_b": 17, "srct_a": 18, "srct_b": 19, "src_a": 20, "src_b": 21}
 
 EXPORTS3D = ["svof3d_create", "svof3d_destroy", "svof3d_field_count", "svof3d_upload_field",
-             "svof3d_download_field", "svof3d_device_field", "svof3d_load_interior", "svof3d_store_interior",
+             "svof3d_download_field", "svof3d_device_field", "svof3d_load_interior", "svof3d_load_interior_device",
+             "svof3d_store_interior",
              "svof3d_load_interior_async", "svof3d_store_interior_async", "svof3d_io_wait",
              "svof3d_fluid_decide_dt", "svof3d_interface_compute_curvature_tensor",
              "svof3d_interface_compute_force", "svof3d_interface_update_vof", "svof3d_fluid_predict_field",
@@ -105,7 +106,7 @@ def lib3() -> ctypes.CDLL:
         L.svof3d_destroy.argtypes = [vp]
         L.svof3d_field_count.argtypes = [vp, i, ctypes.POINTER(sz)]
         for fn in ("svof3d_upload_field", "svof3d_download_field", "svof3d_load_interior", "svof3d_store_interior",
-                   "svof3d_load_interior_async", "svof3d_store_interior_async"):
+                   "svof3d_load_interior_async", "svof3d_store_interior_async", "svof3d_load_interior_device"):
             getattr(L, fn).argtypes = [vp, i, dp, sz]
         L.svof3d_io_wait.argtypes = [vp]
         L.svof3d_statistics_collect.argtypes = [vp]
@@ -265,6 +266,17 @@ class Solver3D:
         if a.shape != want:
             raise ValueError(f"{name}: expected shape {want}, got {a.shape}")
         _check(lib3().svof3d_load_interior(self._h, FIELDS3D[name], a.ctypes.data, a.size))
+
+    def load_interior_device(self, name: str, a):
+        """load_interior from a contiguous float64 CUDA tensor of the field's
+        restart shape (work on torch's current stream is waited for)"""
+        import torch
+        want = interior_shape3d(name, self.nx, self.ny, self.nz)
+        if (not isinstance(a, torch.Tensor) or not a.is_cuda or a.dtype != torch.float64 or tuple(a.shape) != want
+                or not a.is_contiguous()):
+            raise ValueError(f"{name}: expected a contiguous float64 CUDA tensor of shape {want}")
+        torch.cuda.current_stream(a.device).synchronize()
+        _check(lib3().svof3d_load_interior_device(self._h, FIELDS3D[name], a.data_ptr(), a.numel()))
 
     def interior(self, name: str) -> np.ndarray:
         out = np.empty(interior_shape3d(name, self.nx, self.ny, self.nz))
