@@ -25,7 +25,7 @@
 
 #include "svof3d_internal.cuh"
 #include "smem_limit.cuh"
-#include "tdm_pivots.cuh"
+#include "tdm_segments.cuh"
 
 // Precision split as in k3_interface.cu: SVOF3_PRECISION=64 builds the FP64
 // instantiations and the shared code (no FMA contraction), =32 the FP32

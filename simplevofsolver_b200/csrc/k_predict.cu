@@ -7,26 +7,27 @@
 // into src_g), stores src_a for the next substep and keeps the increment
 // delta = dt (alpha src_a + beta src_b + gamma src_g) in shared memory.
 // Phase 2 solves the implicit-x systems (1 - gamma dt nu / 2 Lx) delta' =
-// delta with the Thomas recurrence of src/tdm.c:17-50, one line (field, row)
-// per thread.  Phase 3 writes u + delta' into the other buffer of the
+// delta with the Thomas recurrence of src/tdm.c:17-50, a warp a line (field,
+// row; tdm_segments.cuh).  Phase 3 writes u + delta' into the other buffer of the
 // ping-pong pair together with the halo rows and wall values that
 // fluid_update_boundaries_{ux,uy,t} assign.
 #include <cuda_pipeline.h>
 
 #include "svof_internal.cuh"
-#include "tdm_pivots.cuh"
+#include "tdm_segments.cuh"
 
 namespace svof {
 
-// increments [3][R][nx+1] and the substep's Thomas coefficients [9][nx+1]
+// increments and the sweeps' forward values [3][R][nx+1] each, and the
+// substep's Thomas coefficients [9][nx+1]
 size_t predict_smem_bytes(int nx, int R) {
-  return sizeof(double) * ((size_t)3 * R * (nx + 1) + (size_t)9 * (nx + 1));
+  return sizeof(double) * ((size_t)6 * R * (nx + 1) + (size_t)9 * (nx + 1));
 }
 
 // Thomas coefficients of the three implicit-x systems of one substep
 // (solve_in_x of src/fluid/predict/{ux,uy,t}.c and gtsv, src/tdm.c:17-50):
 // they depend on dt and the substep only, so one warp per field computes
-// them once (tdm_pivots.cuh) and every line solve reads them.  Layout per field f at
+// them once (tdm_segments.cuh) and every line solve reads them.  Layout per field f at
 // coef + 3 f nx:  L[i] = tdm_l[i];  R[0] = tdm_c[0], R[i] = 1 / (c_i - l_i
 // v_{i-1}) for 0 < i < n-1, R[n-1] = 1 / (c - l v) of the last row or 0 when
 // the reference zeroes that row;  V[i] = v_i.
@@ -59,7 +60,9 @@ __global__ void k_tdm_coef(const double *__restrict__ lap_ux, const double *__re
   svof_tdm::pivots(lap, pf, n, L, R, V);
 }
 
-// right-hand sides of ux (i >= 2), uy and t at cell (i, j), exactly as
+// right-hand sides of ux (i >= 2), uy and t at cell (i, j) (the quotients of
+// spacings from tables instead of nine divisions a cell: 512 x 1024 predictor
+// in the line form 84 -> 78 us a substep), exactly as
 // compute_rhs_{ux,uy,t} (src/fluid/predict/{ux,uy,t}.c): src_a is stored for
 // the next substep, the increments dt (alpha src_a + beta src_b + gamma src_g)
 // go to d[0..2] (d[0] only for i >= 2)
@@ -67,30 +70,28 @@ __device__ __forceinline__ void predict_rhs_cell(const PredictArgs &a, int i, in
                                                  double cg, double *d) {
   const Grid2 &g = a.g;
   const int nx = g.nx;
-  const double dy = g.dy;
+  const double hy = a.hdy, rdy = a.rdy;
+  const RhsQuot Q = a.quot[i - 1];
   const double *ux = a.ux, *uy = a.uy, *p = a.p, *t = a.t;
-  const double dxf_i = g.dxf[i - 1];
     // ---- ux at (i, j), i in [2, nx]: compute_rhs_ux, ux.c:218-249
     if (i >= 2) {
-      const double dxc_i = g.dxc[i - 1];
       const double uxm = ux[ix_ux(nx, i - 1, j)], uxc = ux[ix_ux(nx, i, j)], uxp = ux[ix_ux(nx, i + 1, j)];
       const double uxs = ux[ix_ux(nx, i, j - 1)], uxn = ux[ix_ux(nx, i, j + 1)];
       double sa = 0., sg = 0.;
       {  // advection_x, ux.c:71-92
         const double ux_l = +0.5 * uxm + 0.5 * uxc;
         const double ux_u = +0.5 * uxc + 0.5 * uxp;
-        const double l = +0.5 / dxc_i * ux_l;
-        const double u = -0.5 / dxc_i * ux_u;
+        const double l = Q.hxc * ux_l;
+        const double u = -Q.hxc * ux_u;
         const double c = -l - u;
         sa += +l * uxm + c * uxc + u * uxp;
       }
       {  // advection_y, ux.c:94-120
-        const double w_xm = 0.5 * g.dxf[i - 2] / dxc_i;
-        const double w_xp = 0.5 * dxf_i / dxc_i;
+        const double w_xm = Q.w_xm, w_xp = Q.w_xp;
         const double uy_l = w_xm * uy[ix_cc(nx, i - 1, j)] + w_xp * uy[ix_cc(nx, i, j)];
         const double uy_u = w_xm * uy[ix_cc(nx, i - 1, j + 1)] + w_xp * uy[ix_cc(nx, i, j + 1)];
-        const double l = +0.5 / dy * uy_l;
-        const double u = -0.5 / dy * uy_u;
+        const double l = hy * uy_l;
+        const double u = -hy * uy_u;
         const double c = -l - u;
         sa += +l * uxs + c * uxc + u * uxn;
       }
@@ -101,7 +102,7 @@ __device__ __forceinline__ void predict_rhs_cell(const PredictArgs &a, int i, in
       // diffusion_y (explicit, src_a), ux.c:143-161
       sa += a.m_dif * (+a.lapy0 * uxs + a.lapy1 * uxc + a.lapy2 * uxn);
       // pressure (src_g), ux.c:164-179
-      sg -= 1. / dxc_i * (-p[ix_cc(nx, i - 1, j)] + p[ix_cc(nx, i, j)]);
+      sg -= Q.rdxc * (-p[ix_cc(nx, i - 1, j)] + p[ix_cc(nx, i, j)]);
       // buoyancy, ux.c:181-197
       if (a.add_buoyancy) sa += +0.5 * t[ix_cc(nx, i - 1, j)] + 0.5 * t[ix_cc(nx, i, j)];
       // surface, ux.c:199-210
@@ -118,16 +119,16 @@ __device__ __forceinline__ void predict_rhs_cell(const PredictArgs &a, int i, in
       {  // advection_x, uy.c:70-92
         const double ux_l = +0.5 * ux[ix_ux(nx, i, j - 1)] + 0.5 * ux[ix_ux(nx, i, j)];
         const double ux_u = +0.5 * ux[ix_ux(nx, i + 1, j - 1)] + 0.5 * ux[ix_ux(nx, i + 1, j)];
-        const double l = +0.5 / dxf_i * ux_l;
-        const double u = -0.5 / dxf_i * ux_u;
+        const double l = Q.hxf * ux_l;
+        const double u = -Q.hxf * ux_u;
         const double c = -l - u;
         sa += +l * uym + c * uyc + u * uyp;
       }
       {  // advection_y, uy.c:94-115
         const double uy_l = +0.5 * uys + 0.5 * uyc;
         const double uy_u = +0.5 * uyc + 0.5 * uyn;
-        const double l = +0.5 / dy * uy_l;
-        const double u = -0.5 / dy * uy_u;
+        const double l = hy * uy_l;
+        const double u = -hy * uy_u;
         const double c = -l - u;
         sa += +l * uys + c * uyc + u * uyn;
       }
@@ -138,7 +139,7 @@ __device__ __forceinline__ void predict_rhs_cell(const PredictArgs &a, int i, in
       // diffusion_y (src_a), uy.c:138-156
       sa += a.m_dif * (+a.lapy0 * uys + a.lapy1 * uyc + a.lapy2 * uyn);
       // pressure (src_g), uy.c:159-174
-      sg -= 1. / dy * (-p[ix_cc(nx, i, j - 1)] + p[ix_cc(nx, i, j)]);
+      sg -= rdy * (-p[ix_cc(nx, i, j - 1)] + p[ix_cc(nx, i, j)]);
       // surface, uy.c:176-187
       sa += a.ifrcy[ix_src(nx, i, j)];
       // extension: buoyancy of the volume fraction (not in the reference)
@@ -155,14 +156,14 @@ __device__ __forceinline__ void predict_rhs_cell(const PredictArgs &a, int i, in
       const double ts = t[ix_cc(nx, i, j - 1)], tn = t[ix_cc(nx, i, j + 1)];
       double sa = 0., sg = 0.;
       {  // advection_x, t.c:68-89
-        const double l = +0.5 / dxf_i * ux[ix_ux(nx, i, j)];
-        const double u = -0.5 / dxf_i * ux[ix_ux(nx, i + 1, j)];
+        const double l = Q.hxf * ux[ix_ux(nx, i, j)];
+        const double u = -Q.hxf * ux[ix_ux(nx, i + 1, j)];
         const double c = -l - u;
         sa += +l * tm + c * tc + u * tp;
       }
       {  // advection_y, t.c:91-112
-        const double l = +0.5 / dy * uy[ix_cc(nx, i, j)];
-        const double u = -0.5 / dy * uy[ix_cc(nx, i, j + 1)];
+        const double l = hy * uy[ix_cc(nx, i, j)];
+        const double u = -hy * uy[ix_cc(nx, i, j + 1)];
         const double c = -l - u;
         sa += +l * ts + c * tc + u * tn;
       }
@@ -178,23 +179,26 @@ __device__ __forceinline__ void predict_rhs_cell(const PredictArgs &a, int i, in
     }
   }
 
-__global__ void __launch_bounds__(256) k_predict(PredictArgs a) {
+__global__ void __launch_bounds__(256, 3) k_predict(PredictArgs a) {
   pdl_enter();
   extern __shared__ double sm[];
   const Grid2 g = a.g;
   const int nx = g.nx, ny = g.ny, R = a.rows_per_block;
   const int ld = nx + 1;
   double *sd = sm;                  // [3][R][ld] increments
-  double *sc = sm + 3 * R * ld;     // [9][ld] Thomas coefficients (L, R, V of ux, uy, t)
+  double *sq = sd + 3 * R * ld;     // [3][R][ld] the sweeps' forward values
+  double *sc = sq + 3 * R * ld;     // [9][ld] Thomas coefficients (L, R, V of ux, uy, t)
   const int j0 = 1 + blockIdx.x * R;
   const int nrows = min(R, ny - j0 + 1);
   const double dt = *a.dtp;
   const double ca = a.rk.a * dt, cb = a.rk.b * dt, cg = a.rk.g * dt;
   const int tid = threadIdx.x;
 
+#pragma unroll 4
   for (int w = tid; w < 9 * nx; w += blockDim.x) sc[(w / nx) * ld + (w % nx)] = a.coef[w];
 
   // ---------------- phase 1: right-hand sides and increments
+#pragma unroll 2
   for (int w = tid; w < nrows * nx; w += blockDim.x) {
     const int jj = w / nx;
     const int i = 1 + w % nx;
@@ -208,37 +212,16 @@ __global__ void __launch_bounds__(256) k_predict(PredictArgs a) {
   __syncthreads();
 
   // ---------------- phase 2: Thomas sweeps (gtsv, src/tdm.c:17-50) with the
-  // coefficients of k_tdm_coef
-  const bool line = tid < 3 * nrows;
-  if (line) {
-    const int f = tid / nrows;
-    const int jj = tid % nrows;
-    const int n = (0 == f) ? nx - 1 : nx;
-    double *q = sd + (f * R + jj) * ld;
-    const double *L = sc + (3 * f + 0) * ld;
-    const double *Rv = sc + (3 * f + 1) * ld;
-    const double *V = sc + (3 * f + 2) * ld;
-    double qprev = q[0] / Rv[0];
-    q[0] = qprev;
-#pragma unroll 4
-    for (int i = 1; i < n - 1; i++) {
-      qprev = Rv[i] * (q[i] - L[i] * qprev);
-      q[i] = qprev;
-    }
-    {
-      const double rl = Rv[n - 1];
-      q[n - 1] = (0. != rl) ? rl * (q[n - 1] - L[n - 1] * qprev) : 0.;
-    }
-    double qn = q[n - 1];
-#pragma unroll 4
-    for (int i = n - 2; i >= 0; i--) {
-      qn = q[i] - V[i] * qn;
-      q[i] = qn;
-    }
+  // coefficients of k_tdm_coef, a warp a line
+  for (int w = tid >> 5; w < 3 * nrows; w += blockDim.x >> 5) {
+    const int f = w / nrows, jj = w - f * nrows;
+    svof_tdm::line_solve(sc + (3 * f + 0) * ld, sc + (3 * f + 1) * ld, sc + (3 * f + 2) * ld, (0 == f) ? nx - 1 : nx,
+                         sd + (f * R + jj) * ld, sq + (f * R + jj) * ld);
   }
   __syncthreads();
 
   // ---------------- phase 3: u + delta', halo rows and walls
+#pragma unroll 2
   for (int w = tid; w < nrows * (nx + 2); w += blockDim.x) {
     const int r = w / (nx + 2);
     const int c = w % (nx + 2);
@@ -288,9 +271,9 @@ __global__ void __launch_bounds__(256) k_predict(PredictArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// Line-streaming form for large grids: the fused kernel above keeps whole
-// rows in shared memory, so a block holds few rows and its Thomas phase runs
-// few lines per SM (the serial recurrence then sets the time).  Here the
+// Line-streaming form for large grids of long rows: the fused kernel above
+// keeps whole rows and the coefficients of whole lines in shared memory, so
+// long rows leave an SM one block of one or two rows.  Here the
 // right-hand sides of a 32 x 32 tile go to a line array, one warp per field
 // and 32 lines sweeps it (forward and backward) from a ring of shared-memory
 // chunks that cp.async fills ahead, and a tiled pass writes u + delta', the

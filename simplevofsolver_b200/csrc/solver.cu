@@ -217,6 +217,9 @@ int launch_predict(svof_solver *s, int rk, bool with_coef) {
   a.lap_ux = s->lap_ux.p;
   a.lap_uy = s->lap_uy.p;
   a.lap_t = s->lap_t.p;
+  a.quot = reinterpret_cast<const RhsQuot *>(s->quot.p);
+  a.hdy = 0.5 / s->dy;
+  a.rdy = 1. / s->dy;
   a.coef = coef_table(s, rk);
   a.dtp = s->d_dt;
   a.m_dif = s->prm.m_dif;
@@ -458,6 +461,20 @@ int build_tables(svof_solver *s, const double *xf, const double *xc) {
     luy[3 * (i - 1) + 2] = u;
   }
   if (upload(s->lap_ux, lux) || upload(s->lap_uy, luy) || upload(s->lap_t, luy)) return 1;
+  constexpr int nq = sizeof(RhsQuot) / sizeof(double);
+  std::vector<double> quot((size_t)nq * nx);
+  for (int i = 1; i <= nx; i++) {
+    RhsQuot q{};
+    if (i >= 2) {
+      q.hxc = 0.5 / DXC(i);
+      q.rdxc = 1. / DXC(i);
+      q.w_xm = 0.5 * DXF(i - 1) / DXC(i);
+      q.w_xp = 0.5 * DXF(i) / DXC(i);
+    }
+    q.hxf = 0.5 / DXF(i);
+    std::memcpy(&quot[(size_t)nq * (i - 1)], &q, sizeof(q));
+  }
+  if (upload(s->quot, quot)) return 1;
   s->lapy[0] = +1. / s->dy / s->dy;
   s->lapy[1] = -2. / s->dy / s->dy;
   s->lapy[2] = +1. / s->dy / s->dy;
@@ -598,26 +615,46 @@ int engine_create(const svof_params_t *prm, const double *xf, const double *xc, 
   if (cudaSuccess != cudaStreamCreateWithFlags(&s->side2, cudaStreamNonBlocking)) return fail("stream"), bail();
   for (cudaEvent_t *e : s->branch_events())
     if (cudaSuccess != cudaEventCreateWithFlags(e, cudaEventDisableTiming)) return fail("event"), bail();
-  // predict launch shape: R rows per block, enough blocks to cover the SMs,
-  // within 200 KB of shared memory
+  // predict launch shape: rows per block.  A block's time is latency (its
+  // loads about 6 us, a cell a thread 2.2, a line a warp 3), so the rows are
+  // those with the least waves times that, over the blocks an SM holds by
+  // shared memory and registers (three of 256 threads).  us a substep of the
+  // predictor and its tables, against ny / 148 rows: 256^2 28 -> 22, 512^2 49
+  // -> 38, 100 x 1024 34 -> 26, 1024 x 256 110 -> 57.
   {
-    const long per_row = 3L * (nx + 1);
+    const long per_row = 6L * (nx + 1);
     const long fixed = 9L * (nx + 1);
-    long r = std::max(1, std::min(8, ny / 148));
-    while (r > 1 && (fixed + r * per_row) * 8 > 200L * 1024) r--;
-    s->pred_rows = (int)r;
-    s->pred_threads = (r <= 2) ? 128 : 256;
+    auto kb = [&](long r) { return (fixed + r * per_row) * 8 / 1024 + 1; };
+    const bool fits = kb(1) <= 226;  // else the line form, whatever the grid
+    long best = -1;
+    s->pred_rows = 1;
+    for (long r = 1; r <= 8 && (1 == r || kb(r) <= 200); r++) {
+      const long threads = r * nx > 128 ? 256 : 128;
+      const long held = 148 * std::max(1L, std::min(768 / threads, 227 / (kb(r) + 1)));
+      const long blocks = (ny + r - 1) / r;
+      const long us = 60 + 22 * ((r * nx + threads - 1) / threads) + 30 * ((3 * r + threads / 32 - 1) / (threads / 32));
+      const long cost = (blocks + held - 1) / held * us;
+      if (best < 0 || cost < best) {
+        best = cost;
+        s->pred_rows = (int)r;
+        s->pred_threads = (int)threads;
+      }
+    }
     s->pred_smem = predict_smem_bytes(nx, s->pred_rows);
-    if (s->pred_smem > 200 * 1024) return fail("svof_create: nx = %d too large for the x line solver", nx), bail();
-    if (cudaSuccess != raise_smem_limit(k_predict, s->pred_smem))
+    if (12L * 8 * (nx + 1) > 200 * 1024) return fail("svof_create: nx = %d too large for the x line solver", nx), bail();
+    if (fits && cudaSuccess != raise_smem_limit(k_predict, s->pred_smem))
       return fail("cudaFuncSetAttribute(k_predict): %s", cudaGetErrorString(cudaGetLastError())), bail();
     const size_t coef_smem = sizeof(double) * 9 * nx;
     if (cudaSuccess != raise_smem_limit(k_tdm_coef, coef_smem)) return fail("cudaFuncSetAttribute(k_tdm_coef)"), bail();
-    // grids from 512 x 512 cells take the line-streaming predictor: the
-    // fused kernel's row tiles leave few lines per SM for its serial sweeps.
-    // SVOF_PREDICT_LINES = 0 / 1 forces either form (tests compare them).
-    s->pred_lines = (long)nx * ny >= 512L * 512L;
+    // large grids of long rows take the line-streaming predictor: the fused
+    // kernel's blocks then hold an SM each for a row or two.  us a step, fused
+    // against lines: 512^2 302 / 364, 300 x 2048 532 / 574, 512 x 2048 979 /
+    // 979, 1024 x 256 339 / 426, 1024 x 512 589 / 589, 1501 x 512 978 / 820,
+    // 1024^2 1139 / 956.  SVOF_PREDICT_LINES = 0 / 1 forces either form (tests
+    // compare them).
+    s->pred_lines = (long)nx * ny >= 1L << 19 && nx > 768;
     if (const char *e = std::getenv("SVOF_PREDICT_LINES")) s->pred_lines = (0 != std::atoi(e));
+    s->pred_lines |= !fits;
     if (s->pred_lines) {
       if (dalloc(s->fw, 3 * (size_t)nx * 32 * ((ny + 31) / 32))) return bail();
       if (cudaSuccess != raise_smem_limit(k_predict_xsolve, predict_xsolve_smem(nx)))
@@ -654,8 +691,8 @@ int engine_create(const svof_params_t *prm, const double *xf, const double *xc, 
   // launch plan checks: every dynamic shared-memory size covers what the
   // kernel indexes, every line solve has a thread per line
   {
-    const size_t need_pred = sizeof(double) * (3 * (size_t)s->pred_rows + 9) * (nx + 1);
-    if (s->pred_smem < need_pred || s->pred_threads < 3 * s->pred_rows || s->pred_rows < 1)
+    const size_t need_pred = sizeof(double) * (6 * (size_t)s->pred_rows + 9) * (nx + 1);
+    if (s->pred_smem < need_pred || s->pred_rows < 1)
       return fail("svof_create: inconsistent predictor launch plan"), bail();
     if (s->uniform && (s->ysolve_kt < 1 || s->ysolve_kt > 64 || s->ysolve_kt > 128))
       return fail("svof_create: inconsistent y line-solve launch plan"), bail();
@@ -720,7 +757,7 @@ int svof_destroy(svof_solver_t *s) {
     dfree(s->sux[k]); dfree(s->suy[k]); dfree(s->st[k]); dfree(s->svof[k]);
   }
   DevBuf *bufs[] = {&s->p, &s->psi, &s->curv, &s->normal, &s->ifrcx, &s->ifrcy, &s->dxf, &s->dxc,
-                    &s->lap_ux, &s->lap_uy, &s->lap_t, &s->spec, &s->twf, &s->twb, &s->cs, &s->vt,
+                    &s->lap_ux, &s->lap_uy, &s->lap_t, &s->quot, &s->spec, &s->twf, &s->twb, &s->cs, &s->vt,
                     &s->rvt, &s->q1t, &s->ck, &s->lastf, &s->den, &s->pl, &s->pu, &s->evals, &s->diag,
                     &s->coef, &s->stat_part, &s->fw};
   for (DevBuf *b : bufs) dfree(*b);

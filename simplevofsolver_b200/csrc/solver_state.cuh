@@ -41,7 +41,7 @@ struct svof_solver {
   int sa_f = 0;    // which of sux/suy/st[] is src[rk_a]
   int sa_v = 0;    // which of svof[] is src[rk_a]
   // grid tables
-  svof::DevBuf dxf, dxc, lap_ux, lap_uy, lap_t;
+  svof::DevBuf dxf, dxc, lap_ux, lap_uy, lap_t, quot;
   double lapy[3] = {0., 0., 0.};
   double dif_m_y = 0., dif_t_y = 0.;
   // Poisson

@@ -71,12 +71,19 @@ __global__ void k_vof_advect(const double *__restrict__ vof, double *__restrict_
                              RK rk, int use_b, Grid2 g);
 // fused momentum / scalar right-hand sides, increments, implicit-x Thomas
 // sweeps and field update (src/fluid/predict/*.c, src/tdm.c:17-50)
+// quotients of grid spacings of column i (index i - 1), the values of the
+// expressions the reference evaluates per cell (the ux ones from i = 2 on)
+struct RhsQuot {
+  double hxc, rdxc, w_xm, w_xp, hxf, unused;  // 0.5 / dxc, 1 / dxc, 0.5 dxf(i - 1) / dxc, 0.5 dxf / dxc, 0.5 / dxf
+};
 struct PredictArgs {
   const double *ux, *uy, *p, *t, *ifrcx, *ifrcy;
   double *ux_new, *uy_new, *t_new;
   double *sux_a, *suy_a, *st_a;
   const double *sux_b, *suy_b, *st_b;
   const double *lap_ux, *lap_uy, *lap_t;  // 3 per row
+  const RhsQuot *quot;
+  double hdy, rdy;                        // 0.5 / dy, 1 / dy
   const double *coef;                     // k_tdm_coef output, [3 fields][L, R, V][nx]
   const double *dtp;
   double m_dif, t_dif;
