@@ -9,7 +9,10 @@
 //              marches along z with the state planes staged in shared memory
 //              by cp.async one plane ahead; writes src_a and the increments
 //              in a line layout
-//   k3_xsolve  the x lines (ny nz of them, serial recurrences): a block owns
+//   k3_xlines  the x lines (ny nz of them): a few whole lines a warp, in
+//              segments over its lanes, and the updated fields with their halo
+//              images and walls
+//   k3_xsolve  the same for lines too long for that: a block owns
 //              32 lines, walks them in 32-cell chunks forward and backward
 //              with one line per lane of four sweeping warps, and writes the
 //              updated fields with their halo images and walls
@@ -669,6 +672,140 @@ __global__ void __launch_bounds__(256) k3_xsolve(Predict3Args<R> a) {
   }
 }
 
+// ---------------------------------------------------------------------------
+// k3_xlines: the same sweeps and update with whole lines on chip.  A warp takes
+// XLB lines of one field at a time (persistent blocks, consecutive warps on
+// consecutive lines) and solves them with XLP lanes a line, each a segment
+// (tdm_segments.cuh); the increments are read once and nothing goes back
+// between the sweeps, 96 bytes a cell instead of k3_xsolve's 160 (FP64), and
+// the chain is a segment's, not a line's.  Shared memory: the three systems'
+// tables and the lines.  A warp's phases (loads, solve, update) follow one
+// another, so warps in flight are what hides them; fewer lanes a line cost
+// fewer instructions but leave an SM fewer warps.  Measured best: 16 lanes and
+// 16 warps on long lines (512: 8 lanes 3.6 ms, 16 lanes 2.7, 16 lanes and 20
+// warps 3.2), 8 lanes and 24 warps below.  ms a launch, against k3_xsolve:
+// 512^3 FP64 2.7 / 4.5 (4.8 TB/s), mixed 2.3 / 3.6, 256^3 FP64 0.41 / 0.57.
+struct XlLong {
+  static constexpr int XLP = 16, MAXW = 16;
+};
+struct XlShort {
+  static constexpr int XLP = 8, MAXW = 24;
+};
+constexpr int kXlLongFrom = 321;  // cells a line
+// rows ahead of a segment
+template <class R>
+constexpr int kXlWarm = 4 == sizeof(R) ? 16 : 24;
+// rows a lane (odd) and a line's pitch: the lanes of a half warp (a warp, FP32),
+// on rows s seg + k of lines m, fall on distinct banks when the pitch is
+// XLP seg modulo 16 (32)
+template <class S>
+__host__ __device__ constexpr int xl_seg(int nx) {
+  return ((nx - 2 + S::XLP - 1) / S::XLP) | 1;
+}
+template <class R, class S>
+__host__ __device__ constexpr int xl_pitch(int nx) {
+  constexpr int m = 128 / (int)sizeof(R);
+  return nx + ((S::XLP * xl_seg<S>(nx) - nx) % m + m) % m;
+}
+template <class R, class S>
+__host__ __device__ constexpr size_t xl_warp_bytes(int nx) {
+  return 32 / S::XLP * sizeof(R) * (size_t)xl_pitch<R, S>(nx);
+}
+template <class R>
+__host__ __device__ constexpr size_t xl_table_bytes(int nx) {
+  return (9 * sizeof(R) * (size_t)(nx | 1) + 15) / 16 * 16;
+}
+
+// the L2 lines of [p, p + bytes), a warp
+__device__ __forceinline__ void prefetch_l2(const void *p, long bytes, int lane) {
+  for (long o = 128 * lane; o < bytes; o += 128 * 32)
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char *>(p) + o));
+}
+
+template <class R, class S>
+__global__ void __launch_bounds__(S::MAXW * 32) k3_xlines(Predict3Args<R> a) {
+  using T = SweepT<R>;
+  constexpr int XLP = S::XLP, XLB = 32 / XLP;
+  extern __shared__ double smd[];
+  const Grid3 g = a.g;
+  const int nx = g.nx, ny = g.ny, nz = g.nz, lt = nx | 1, ld = xl_pitch<R, S>(nx);
+  T *co = reinterpret_cast<T *>(smd);  // [9][lt]: L, R, V of the three systems
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  R *x = reinterpret_cast<R *>(reinterpret_cast<char *>(smd) + xl_table_bytes<R>(nx)) + (size_t)XLB * ld * warp;
+  const long nlines = (long)ny * nz, ntask = 4 * nlines / XLB;  // ny, nz powers of two, at least 4: whole tasks
+  for (int w = threadIdx.x; w < 9 * nx; w += blockDim.x) co[(w / nx) * lt + w % nx] = T(ldg(a.coef + w));
+  __syncthreads();
+  for (long t = (long)blockIdx.x * nw + warp; t < ntask; t += (long)gridDim.x * nw) {
+    const int f = (int)(XLB * t / nlines);
+    const long l0 = XLB * t - f * nlines;
+    const int set = (0 == f) ? 0 : (3 == f ? 2 : 1), n = (0 == f) ? nx - 1 : nx;
+    const R *src = a.fw + ((size_t)f * nlines + l0) * nx;
+    for (int m = 0; m < XLB; m++)
+#pragma unroll 8
+      for (int p = lane; p < n; p += 32)
+        __pipeline_memcpy_async(x + m * ld + p, src + (size_t)m * nx + p, sizeof(R));
+    __pipeline_commit();
+    // storage rows of the field: position p of the line at column p + 1.  The
+    // lines of a task lie in one plane (ny is a multiple of XLB)
+    const double *u = 0 == f ? a.ux : (1 == f ? a.uy : (2 == f ? a.uz : a.t));
+    double *un = 0 == f ? a.ux_new : (1 == f ? a.uy_new : (2 == f ? a.uz_new : a.t_new));
+    const long pitch = (0 == f) ? nx + 1 : nx + 2;
+    auto row = [&](int jj, int kk) { return pitch * (jj + (long)(ny + 2) * kk); };
+    const int j0 = 1 + (int)(l0 % ny), k = 1 + (int)(l0 / ny);
+    // into L2 while the lines are solved: their fields' rows (512^3 FP64 2.7
+    // ms a launch, 3.1 without) and, for FP32 increments, the next task's
+    // (2.3, 2.7 without; FP64 gains nothing)
+    prefetch_l2(u + row(j0, k), XLB * pitch * sizeof(double), lane);
+    const long t1 = t + (long)gridDim.x * nw;
+    if (4 == sizeof(R) && 16 == XLP && t1 < ntask) prefetch_l2(a.fw + (size_t)XLB * t1 * nx, XLB * nx * sizeof(R), lane);
+    __pipeline_wait_prior(0);
+    __syncwarp();
+    const int m_ = lane / XLP;
+    svof_tdm::group_solve<T, XLP, kXlWarm<R>>(co + 3 * set * lt, co + (3 * set + 1) * lt, co + (3 * set + 2) * lt, n,
+                                              xl_seg<S>(nx), x + m_ * ld, src + (size_t)m_ * nx);
+    const double lo = 0 == f ? 0. : (1 == f ? a.uy_xm : (2 == f ? a.uz_xm : a.t_xm));
+    const double hi = 0 == f ? 0. : (1 == f ? a.uy_xp : (2 == f ? a.uz_xp : a.t_xp));
+    for (int m = 0; m < XLB; m++) {
+      const int j = j0 + m;
+      const long o = row(j, k) + 1;
+#pragma unroll 16
+      for (int p = lane; p < n; p += 32) un[o + p] = ldg(u + o + p) + x[m * ld + p];
+      if (1 == j || ny == j || 1 == k || nz == k) {
+        for (int p = lane; p < n; p += 32) {
+          const double v = ldg(u + o + p) + x[m * ld + p];
+          for_images(j, k, ny, nz, false, [&](int jj, int kk) { un[row(jj, kk) + p + 1] = v; });
+        }
+      }
+    }
+    // walls: the halo images take the value before the wall assignment
+    if (lane < 2 * XLB) {
+      const int j = j0 + (lane >> 1);
+      const long c = (lane & 1) ? pitch - 1 : 0;
+      const double old = ldg(u + row(j, k) + c);
+      un[row(j, k) + c] = (lane & 1) ? hi : lo;
+      for_images(j, k, ny, nz, false, [&](int jj, int kk) { un[row(jj, kk) + c] = old; });
+    }
+    __syncwarp();  // the lines' buffers are free
+  }
+}
+
+// warps of a k3_xlines block: what fits an SM, no more than there is work for;
+// 0 where fewer than 8 fit (x lines of more than about 1150 FP64 cells:
+// k3_xsolve).  Against k3_xsolve at the small end: 61 x 64 x 32 four steps 1002
+// / 1080 us, 128^3 mixed stream 8.71 / 8.74 ms.
+template <class R, class S>
+int xlines_warps(int nx, long nlines) {
+  const long room = 226L * 1024 - (long)xl_table_bytes<R>(nx);
+  const long fit = room / (long)xl_warp_bytes<R, S>(nx);
+  if (fit < 8) return 0;
+  return (int)std::min({(long)S::MAXW, fit, std::max(2L, (4 * nlines * S::XLP / 32 + 147) / 148)});
+}
+// f(shape) for lines of nx cells
+template <class F>
+cudaError_t by_xl_shape(int nx, F f) {
+  return nx >= kXlLongFrom ? f(XlLong()) : f(XlShort());
+}
+
 template <class R>
 cudaError_t predict_launch(cudaStream_t st, const Predict3Args<R> &a) {
   const Grid3 &g = a.g;
@@ -679,33 +816,49 @@ cudaError_t predict_launch(cudaStream_t st, const Predict3Args<R> &a) {
   cudaError_t e = cudaGetLastError();
   if (cudaSuccess != e) return e;
   const long nlines = (long)g.ny * g.nz;
-  k3_xsolve<R><<<(unsigned)((nlines + PL - 1) / PL), 256, 0, st>>>(a);
-  return cudaGetLastError();
+  return by_xl_shape(g.nx, [&](auto shape) {
+    using S = decltype(shape);
+    const int nw = xlines_warps<R, S>(g.nx, nlines);
+    if (nw > 0) {
+      const unsigned blocks = (unsigned)std::min<long>(148, (4 * nlines * S::XLP / 32 + nw - 1) / nw);
+      k3_xlines<R, S><<<blocks, 32 * nw, xl_table_bytes<R>(g.nx) + nw * xl_warp_bytes<R, S>(g.nx), st>>>(a);
+    } else {
+      k3_xsolve<R><<<(unsigned)((nlines + PL - 1) / PL), 256, 0, st>>>(a);
+    }
+    return cudaGetLastError();
+  });
 }
 
 template <class R>
-cudaError_t predict_prepare_t() {
-  const cudaError_t e = raise_smem_limit(k3_rhs<R, false>, kRhsSmem<R>);
+cudaError_t predict_prepare_t(int nx, long nlines) {
+  cudaError_t e = raise_smem_limit(k3_rhs<R, false>, kRhsSmem<R>);
+  if (cudaSuccess != e) return e;
+  e = by_xl_shape(nx, [&](auto shape) {
+    using S = decltype(shape);
+    const int nw = xlines_warps<R, S>(nx, nlines);
+    return nw > 0 ? raise_smem_limit(k3_xlines<R, S>, xl_table_bytes<R>(nx) + nw * xl_warp_bytes<R, S>(nx))
+                  : cudaSuccess;
+  });
   if (cudaSuccess != e) return e;
   return raise_smem_limit(k3_rhs<R, true>, kRhsSmem<R>);
 }
 #if SVOF3_WITH_F64
 template cudaError_t predict_launch<double>(cudaStream_t, const Predict3Args<double> &);
-template cudaError_t predict_prepare_t<double>();
+template cudaError_t predict_prepare_t<double>(int, long);
 #endif
 #if SVOF3_WITH_F32
 template cudaError_t predict_launch<float>(cudaStream_t, const Predict3Args<float> &);
-template cudaError_t predict_prepare_t<float>();
+template cudaError_t predict_prepare_t<float>(int, long);
 #endif
 
 #if SVOF3_WITH_F64
 #if !SVOF3_WITH_F32
-extern template cudaError_t predict_prepare_t<float>();
+extern template cudaError_t predict_prepare_t<float>(int, long);
 #endif
-cudaError_t predict_prepare() {
-  cudaError_t e = predict_prepare_t<double>();
+cudaError_t predict_prepare(int nx, long nlines) {
+  cudaError_t e = predict_prepare_t<double>(nx, nlines);
   if (cudaSuccess != e) return e;
-  return predict_prepare_t<float>();
+  return predict_prepare_t<float>(nx, nlines);
 }
 #endif
 

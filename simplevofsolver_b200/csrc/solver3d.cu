@@ -742,7 +742,7 @@ int svof3d_create(const svof3d_params_t *prm, const double *xf, const double *xc
   {
     const cudaError_t pe =
         s->dc ? pois_prepare<float>(s->nx, s->log2ny, s->log2nz) : pois_prepare<double>(s->nx, s->log2ny, s->log2nz);
-    if (cudaSuccess != pe || cudaSuccess != predict_prepare() || cudaSuccess != interface_prepare())
+    if (cudaSuccess != pe || cudaSuccess != predict_prepare(s->nx, (long)s->ny * s->nz) || cudaSuccess != interface_prepare())
       return fail("cudaFuncSetAttribute(Poisson): %s", cudaGetErrorString(cudaGetLastError())), bail();
     const size_t coef_smem = sizeof(double) * 6 * nx;
     if (coef_smem > 200 * 1024) return fail("svof3d_create: nx too large"), bail();

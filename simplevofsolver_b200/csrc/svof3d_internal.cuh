@@ -143,8 +143,8 @@ struct Predict3Args {
 };
 template <class R>
 cudaError_t predict_launch(cudaStream_t st, const Predict3Args<R> &a);
-// opt-in shared memory of the right-hand-side kernel (once per device)
-cudaError_t predict_prepare();
+// opt-in shared memory of the predictor's kernels (lines of nx cells; once per device)
+cudaError_t predict_prepare(int nx, long nlines);
 // Thomas coefficients of up to three substeps for the three distinct systems,
 // one block a substep
 struct Gam3 {

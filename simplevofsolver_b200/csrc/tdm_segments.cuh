@@ -83,23 +83,30 @@ __device__ __forceinline__ void pivots(const double *lap, double pf, int n, doub
   }
 }
 
+__device__ __forceinline__ bool same_bits(double a, double b) {
+  return __double_as_longlong(a) == __double_as_longlong(b);
+}
+__device__ __forceinline__ bool same_bits(float a, float b) { return __float_as_int(a) == __float_as_int(b); }
+
 // gtsv of one line (src/tdm.c:17-50) on the table above: x[0 .. n-1] holds the
 // right-hand side and takes the solution, q[0 .. n-1] is scratch; both and the
 // table in shared memory.  All 32 lanes of the warp take part (n >= 3).
-__device__ __forceinline__ void line_solve(const double *L, const double *R, const double *V, int n, double *x,
-                                           double *q) {
+// WARM: rows ahead (float needs fewer)
+template <class T, int WARM = kWarm>
+__device__ __forceinline__ void line_solve(const T *__restrict__ L, const T *__restrict__ R, const T *__restrict__ V,
+                                           int n, T *__restrict__ x, T *__restrict__ q) {
   const int lane = threadIdx.x & 31;
   const int seg = ((n - 2 + 31) / 32) | 1;  // odd: the lanes' rows on distinct banks
   // ---- forward, x -> q: rows 1 .. n-2 by segments
   {
     const int a = 1 + lane * seg, b = min(a + seg, n - 1);
-    const double q0 = x[0] / R[0];
-    int i = max(1, a - kWarm);
-    double v = (1 == i) ? q0 : 0.;
+    const T q0 = x[0] / R[0];
+    int i = max(1, a - WARM);
+    T v = (1 == i) ? q0 : T(0.);
     const int e = min(a, n - 1);
 #pragma unroll 4
     for (; i < e; i++) v = R[i] * (x[i] - L[i] * v);
-    double start = v;
+    T start = v;
     bool todo = a < b;
     while (__any_sync(0xffffffffu, todo)) {
       if (todo) {
@@ -110,14 +117,14 @@ __device__ __forceinline__ void line_solve(const double *L, const double *R, con
           q[i] = v;
         }
       }
-      const double before = __shfl_up_sync(0xffffffffu, v, 1);
-      todo = a < b && lane > 0 && __double_as_longlong(before) != __double_as_longlong(start);
+      const T before = __shfl_up_sync(0xffffffffu, v, 1);
+      todo = a < b && lane > 0 && !same_bits(before, start);
       if (todo) start = before;
     }
     if (0 == lane) q[0] = q0;
     if (a < b && b == n - 1) {
-      const double r = R[n - 1];
-      q[n - 1] = (0. != r) ? r * (x[n - 1] - L[n - 1] * v) : 0.;
+      const T r = R[n - 1];
+      q[n - 1] = (T(0.) != r) ? r * (x[n - 1] - L[n - 1] * v) : T(0.);
     }
   }
   __syncwarp();
@@ -125,13 +132,13 @@ __device__ __forceinline__ void line_solve(const double *L, const double *R, con
   {
     const int seg_b = ((n - 1 + 31) / 32) | 1;
     const int a = n - 2 - lane * seg_b, b = max(a - seg_b, -1);  // rows a, a - 1 .. b + 1
-    const double qn = q[n - 1];
-    int i = min(n - 2, a + kWarm);
-    double v = (n - 2 == i) ? qn : 0.;
+    const T qn = q[n - 1];
+    int i = min(n - 2, a + WARM);
+    T v = (n - 2 == i) ? qn : T(0.);
     const int e = max(a, -1);
 #pragma unroll 4
     for (; i > e; i--) v = q[i] - V[i] * v;
-    double start = v;
+    T start = v;
     bool todo = a > b;
     while (__any_sync(0xffffffffu, todo)) {
       if (todo) {
@@ -142,12 +149,126 @@ __device__ __forceinline__ void line_solve(const double *L, const double *R, con
           x[i] = v;
         }
       }
-      const double before = __shfl_up_sync(0xffffffffu, v, 1);
-      todo = a > b && lane > 0 && __double_as_longlong(before) != __double_as_longlong(start);
+      const T before = __shfl_up_sync(0xffffffffu, v, 1);
+      todo = a > b && lane > 0 && !same_bits(before, start);
       if (todo) start = before;
     }
     if (0 == lane) x[n - 1] = qn;
   }
+  __syncwarp();
+}
+
+// The same for 32 / LPL lines of a warp at once, LPL lanes a line, in place:
+// x[0 .. n-1] is the line of the calling lane (its group's), src its right-hand
+// side in global memory, read again only by lanes that have to repeat their
+// rows.  seg: rows a lane, odd, LPL seg >= n - 2.  Fewer, longer segments
+// spend less on the rows ahead; rows go in batches, operands first, since a
+// lane's stores are to the array it loads from.
+template <class T, int LPL, int WARM, class R>
+__device__ __forceinline__ void group_solve(const T *__restrict__ L, const T *__restrict__ Rv,
+                                            const T *__restrict__ V, int n, int seg, T *x, const R *src) {
+  constexpr int B = 8;
+  const int s = threadIdx.x & (LPL - 1);
+  const int a = 1 + s * seg, b = min(a + seg, n - 1);
+  const bool has = a < b;
+  T v, start, sb, before;
+  // rows a .. b-1 forward from v, stored
+  auto forward = [&]() {
+    int i = a;
+    for (; i + B <= b; i += B) {
+      T y[B], r[B], l[B];
+#pragma unroll
+      for (int k = 0; k < B; k++) {
+        y[k] = x[i + k];
+        r[k] = Rv[i + k];
+        l[k] = L[i + k];
+      }
+#pragma unroll
+      for (int k = 0; k < B; k++) {
+        v = r[k] * (y[k] - l[k] * v);
+        x[i + k] = v;
+      }
+    }
+    for (; i < b; i++) {
+      v = Rv[i] * (x[i] - L[i] * v);
+      x[i] = v;
+    }
+  };
+  auto backward = [&]() {
+    int i = b - 1;
+    for (; i - B + 1 >= a; i -= B) {
+      T y[B], w[B];
+#pragma unroll
+      for (int k = 0; k < B; k++) {
+        y[k] = x[i - k];
+        w[k] = V[i - k];
+      }
+#pragma unroll
+      for (int k = 0; k < B; k++) {
+        v = y[k] - w[k] * v;
+        x[i - k] = v;
+      }
+    }
+    for (; i >= a; i--) {
+      v = x[i] - V[i] * v;
+      x[i] = v;
+    }
+  };
+  // ---- forward
+  const T q0 = x[0] / Rv[0];
+  {
+    int i = max(1, a - WARM);
+    v = (1 == i) ? q0 : T(0.);
+    const int e = min(a, n - 1);
+#pragma unroll 8
+    for (; i < e; i++) v = Rv[i] * (x[i] - L[i] * v);
+  }
+  __syncwarp();  // the rows ahead are read before their lanes write them
+  start = v;
+  if (has) forward();
+  while (true) {
+    before = __shfl_up_sync(0xffffffffu, v, 1, LPL);
+    const bool again = has && s > 0 && !same_bits(before, start);
+    if (!__any_sync(0xffffffffu, again)) break;
+    if (again) {
+      for (int i = a; i < b; i++) x[i] = T(src[i]);
+      v = start = before;
+      forward();
+    }
+  }
+  if (0 == s) x[0] = q0;
+  if (has && b == n - 1) {
+    const T r = Rv[n - 1];
+    x[n - 1] = (T(0.) != r) ? r * (x[n - 1] - L[n - 1] * v) : T(0.);
+  }
+  __syncwarp();
+  // ---- backward
+  {
+    int i = min(n - 2, b - 1 + WARM);
+    v = (n - 2 == i) ? x[n - 1] : T(0.);
+    if (has) {
+#pragma unroll 8
+      for (; i >= b; i--) v = x[i] - V[i] * v;
+    }
+  }
+  __syncwarp();
+  sb = v;
+  if (has) backward();
+  while (true) {
+    before = __shfl_down_sync(0xffffffffu, v, 1, LPL);
+    const bool again = has && b != n - 1 && !same_bits(before, sb);
+    if (!__any_sync(0xffffffffu, again)) break;
+    if (again) {
+      // the forward values of these rows again, then back from the
+      // neighbour's value
+      for (int i = a; i < b; i++) x[i] = T(src[i]);
+      v = start;
+      forward();
+      v = sb = before;
+      backward();
+    }
+  }
+  if (0 == s) x[0] = x[0] - V[0] * v;
   __syncwarp();
 }
 
