@@ -80,7 +80,7 @@ ALG_WORDS = {
     "poisson_inv": 2.0,        # R spectrum; W psi
     "project": 7.0,            # R psi ux uy p; W ux uy p
 }
-KERNELS_PER_STEP = 2 + 3 * 9  # dt (2), then per substep: coef, geom, force, vof, predict, 3 Poisson, project
+KERNELS_PER_STEP = 3 + 3 * 8  # dt (2), coef, then per substep: geom, force, vof, predict, 3 Poisson, project
 
 # 3D FP64: the ideal dataflow's compulsory 8-byte words per cell-step (145:
 # per substep interface 10, momentum + scalar 20, Poisson 4 + 2 + 2 + 2 + 9,
@@ -107,10 +107,10 @@ ALG_BYTES_3D_MIXED = {
     "predict": 40.0 + 12.0 + 32.0 / 3.0 + 32.0 + 16.0,
     "poisson_fwd": 32.0, "poisson_z": 16.0, "poisson_solve": 16.0, "poisson_inv": 16.0, "project": 72.0,
 }
-# dt (2), then per substep: geom + intercept, force, vof, coef + rhs +
-# line solve, 6 Poisson launches (right-hand side, y, z, x, z, y), project;
-# the same in both paths
-KERNELS_PER_STEP_3D = 2 + 3 * 14
+# dt (2), coef, then per substep: geom + intercept, force, vof, rhs + line
+# solve, 6 Poisson launches (right-hand side, y, z, x, z, y), project; the same
+# in both paths
+KERNELS_PER_STEP_3D = 3 + 3 * 13
 # kernels launched per launch of a kind (profile counts kernels)
 KERNELS_PER_KIND_3D = {"dt": 2, "geom": 2, "predict": 3, "poisson_fwd": 2}
 KERNELS_PER_STEP_3D_MIXED = KERNELS_PER_STEP_3D
