@@ -513,23 +513,35 @@ int build_tables(svof_solver *s, const double *xf, const double *xc) {
         den(nx), lastf(nx);
     const double signal_length = 2. * nx;
     const double gridsize = s->prm.lx / nx;
-    for (size_t k = 0; k < (size_t)nx; k++) {
-      const double ev = -4. / std::pow(gridsize, 2.) * std::pow(std::sin(kGPi * k / signal_length), 2.);
-      for (int r = 0; r < n; r++) c[r] = -l[r] - u[r] + ev;
-      for (int i = 0; i < n - 1; i++) q1[i] = i == 0 ? -l[i] : i == n - 2 ? -u[i] : 0.;
-      host_gtsv(n - 1, l.data(), c.data(), u.data(), v.data(), q1.data());
+    // (columns k in tiles of KT, so that the tables' rows are written in runs)
+    constexpr size_t KT = 8;
+    std::vector<double> tv((size_t)n * KT), tr((size_t)n * KT), tq((size_t)n * KT);
+    for (size_t k0 = 0; k0 < (size_t)nx; k0 += KT) {
+      const size_t kw = std::min(KT, (size_t)nx - k0);
+      for (size_t w = 0; w < kw; w++) {
+        const size_t k = k0 + w;
+        const double ev = -4. / std::pow(gridsize, 2.) * std::pow(std::sin(kGPi * k / signal_length), 2.);
+        for (int r = 0; r < n; r++) c[r] = -l[r] - u[r] + ev;
+        for (int i = 0; i < n - 1; i++) q1[i] = i == 0 ? -l[i] : i == n - 2 ? -u[i] : 0.;
+        host_gtsv(n - 1, l.data(), c.data(), u.data(), v.data(), q1.data());
+        for (int i = 0; i < n - 1; i++) {
+          tv[(size_t)i * KT + w] = v[i];
+          tq[(size_t)i * KT + w] = q1[i];
+        }
+        // gtsv's val of the size-(n-1) system, rows 1 .. n-3, and its last row
+        for (int i = 1; i < n - 2; i++) tr[(size_t)i * KT + w] = 1. / (c[i] - l[i] * v[i - 1]);
+        {
+          const double val = c[n - 2] - l[n - 2] * v[n - 3];
+          lastf[k] = std::fabs(val) > kDblEpsilon ? 1. / val : 0.;
+        }
+        ck[k] = c[0];
+        den[k] = c[n - 1] + u[n - 1] * q1[0] + l[n - 1] * q1[n - 2];
+      }
       for (int i = 0; i < n - 1; i++) {
-        vt[(size_t)i * nx + k] = v[i];
-        q1t[(size_t)i * nx + k] = q1[i];
+        std::memcpy(&vt[(size_t)i * nx + k0], &tv[(size_t)i * KT], sizeof(double) * kw);
+        std::memcpy(&q1t[(size_t)i * nx + k0], &tq[(size_t)i * KT], sizeof(double) * kw);
+        if (i >= 1 && i < n - 2) std::memcpy(&rvt[(size_t)i * nx + k0], &tr[(size_t)i * KT], sizeof(double) * kw);
       }
-      // gtsv's val of the size-(n-1) system, rows 1 .. n-3, and its last row
-      for (int i = 1; i < n - 2; i++) rvt[(size_t)i * nx + k] = 1. / (c[i] - l[i] * v[i - 1]);
-      {
-        const double val = c[n - 2] - l[n - 2] * v[n - 3];
-        lastf[k] = std::fabs(val) > kDblEpsilon ? 1. / val : 0.;
-      }
-      ck[k] = c[0];
-      den[k] = c[n - 1] + u[n - 1] * q1[0] + l[n - 1] * q1[n - 2];
     }
     if (upload(s->vt, vt) || upload(s->rvt, rvt) || upload(s->q1t, q1t) || upload(s->ck, ck) ||
         upload(s->den, den) || upload(s->lastf, lastf))
