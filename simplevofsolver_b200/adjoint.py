@@ -47,21 +47,11 @@ def _interior(a, shape):
     return out
 
 
-class _Held:
-    """The initial p and t of every rollout, held on the GPU: read back as
-    (read-only) arrays in the restart layout, replaced by assignment."""
-
-    def __set_name__(self, owner, name):
-        self.key = "_dev_" + name
-
-    def __get__(self, r, owner=None):
-        a = getattr(r, self.key).cpu().numpy()
-        a.flags.writeable = False
-        return a
-
-    def __set__(self, r, a):
-        import torch
-        setattr(r, self.key, torch.from_numpy(np.array(a, dtype=np.float64)).to("cuda"))
+def _pinned(a):
+    """a copy of the array in page-locked memory (its loads then run at the
+    link's rate)"""
+    import torch
+    return torch.from_numpy(a).pin_memory().numpy()
 
 
 class Rollout:
@@ -72,7 +62,6 @@ class Rollout:
     ``checkpoint_every`` = K."""
 
     STATE = ("ux", "uy", "p", "t", "vof")
-    p0, t0 = _Held(), _Held()
 
     def __init__(self, solver: Solver, dts, checkpoint_every: int = 20, project_initial: bool = True):
         import torch
@@ -82,8 +71,8 @@ class Rollout:
         self.dts = [float(x) for x in dts]
         self.K = int(checkpoint_every)
         self.nx, self.ny = solver.nx, solver.ny
-        self.p0 = solver.interior("p")
-        self.t0 = solver.interior("t")
+        self.p0 = _pinned(solver.interior("p"))
+        self.t0 = _pinned(solver.interior("t"))
         self.tapes = None
         self.checkpoints = []
         self.project = bool(project_initial)
@@ -101,8 +90,8 @@ class Rollout:
             s.set_gravity(float(grav), s.gravity[1])
         for name, a in (("ux", ux0), ("uy", uy0), ("vof", vof0)):
             s.load_interior_device(name, _interior(a, interior_shape(name, self.nx, self.ny)))
-        s.load_interior_device("p", self._dev_p0)
-        s.load_interior_device("t", self._dev_t0)
+        s.load_interior("p", self.p0)
+        s.load_interior("t", self.t0)
         if self.project:
             # the discrete projection u - grad L^-1 div u of the initial
             # velocity (the Poisson solve and correction of a substep; the
@@ -236,7 +225,6 @@ class Rollout3D:
     nx-1), cells (nz, ny, nx)."""
 
     STATE = ("ux", "uy", "uz", "p", "t", "vof")
-    p0, t0 = _Held(), _Held()
 
     def __init__(self, solver, dts, checkpoint_every: int = 20, project_initial: bool = True):
         import torch
@@ -246,8 +234,8 @@ class Rollout3D:
         self.dts = [float(x) for x in dts]
         self.K = int(checkpoint_every)
         self.nx, self.ny, self.nz = solver.nx, solver.ny, solver.nz
-        self.p0 = solver.interior("p")
-        self.t0 = solver.interior("t")
+        self.p0 = _pinned(solver.interior("p"))
+        self.t0 = _pinned(solver.interior("t"))
         self.tapes = None
         self.checkpoints = []
         self.project = bool(project_initial)
@@ -266,8 +254,8 @@ class Rollout3D:
             if tuple(a.shape[:2]) != (self.nz, self.ny):
                 raise ValueError(f"{name}: expected {self.nz} planes of {self.ny} rows, got {tuple(a.shape)}")
             s.load_interior_device(name, _interior(a, interior_shape3d(name, self.nx, self.ny, self.nz)))
-        s.load_interior_device("p", self._dev_p0)
-        s.load_interior_device("t", self._dev_t0)
+        s.load_interior("p", self.p0)
+        s.load_interior("t", self.t0)
         if self.project:
             s.fluid_compute_potential_dft(0, 1.0)
             s.fluid_correct_velocity(0, 1.0)
