@@ -39,11 +39,18 @@ from . import Solver, SvofError, interior_shape, interior_shape3d
 
 
 def _interior(a, shape):
-    """compact (tensor) -> restart layout of the given shape on the GPU, the
-    walls zero"""
+    """compact (tensor, or one that broadcasts to it) -> restart layout of the
+    given shape on the GPU, the walls zero"""
     import torch
     out = torch.zeros(shape, dtype=torch.float64, device="cuda")
-    out[..., 1:-1].copy_(a.detach())
+    inner, a = out[..., 1:-1], a.detach()
+    while a.dim() > inner.dim() and 1 == a.shape[0]:
+        a = a[0]
+    try:
+        a = a.expand(inner.shape)
+    except RuntimeError as e:
+        raise ValueError(f"expected shape {tuple(inner.shape)}: {e}") from None
+    inner.copy_(a)
     return out
 
 
