@@ -611,16 +611,19 @@ cudaError_t line_attrs(K kernel, int smem) {
 // latency, not the bytes, is then what counts) and k3_pois_x streams near the
 // copy rate.  us a launch, whole lines against k3_pois_x: 61 x 64 x 32 10 /
 // 28, 128^3 18 / 53, 256^3 (6 rounds) 116 / 153, 512^3 (44) 1300 / 955.
-static bool pois_x_whole_lines(long nlines, int nx) {
+static size_t pois_x_block_bytes(long nlines, int nx) {
+  return svof_cline::cline_smem(svof_cline::cline_lpb(nlines, nx, sizeof(double)), nx, sizeof(double)) + 1024;
+}
+bool pois_x_fits(long nlines, int nx) { return pois_x_block_bytes(nlines, nx) <= 227 * 1024; }
+bool pois_x_whole_lines(long nlines, int nx) {
+  if (!pois_x_fits(nlines, nx)) return false;
   const int lpb = svof_cline::cline_lpb(nlines, nx, sizeof(double));
-  const size_t bytes = svof_cline::cline_smem(lpb, nx, sizeof(double)) + 1024;
-  if (bytes > 227 * 1024) return false;
-  const long held = 148L * lpb * std::min<long>(32, 227 * 1024 / bytes);
+  const long held = 148L * lpb * std::min<long>(32, 227 * 1024 / pois_x_block_bytes(nlines, nx));
   return nlines <= 12 * held;
 }
 
 template <class R>
-cudaError_t pois_prepare(int nx, int log2ny, int log2nz) {
+cudaError_t pois_prepare(int nx, int log2ny, int log2nz, bool whole_lines) {
   if (log2ny < kMinL2N || log2ny > kMaxL2N || log2nz < kMinL2N || log2nz > kMaxL2N) return cudaErrorInvalidValue;
   cudaError_t e = by_l2n(log2ny, [&](auto c) {
     constexpr int L2 = decltype(c)::value;
@@ -641,7 +644,7 @@ cudaError_t pois_prepare(int nx, int log2ny, int log2nz) {
   });
   if (cudaSuccess != e) return e;
   const long nlines = (long)((1 << log2ny) / 2 + 1) << log2nz;
-  if (pois_x_whole_lines(nlines, nx)) return svof_cline::cline_prepare<R>(nlines, nx);
+  if (whole_lines) return svof_cline::cline_prepare<R>(nlines, nx);
   if (cudaSuccess != (e = line_attrs(k3_pois_x<R, 64>, (int)XShape<R, 64>::SMEM))) return e;
   return line_attrs(k3_pois_x<R, 128>, (int)XShape<R, 128>::SMEM);
 }
@@ -678,7 +681,6 @@ cudaError_t pois_x_table(cudaStream_t st, double *tab, const double *pl, const d
   using namespace svof_cline;
   const int nky = g.ny / 2 + 1;
   const long nlines = (long)nky * g.nz;
-  if (!pois_x_whole_lines(nlines, g.nx)) return cudaSuccess;
   k_cline_table<<<(unsigned)((nlines + kTabLines - 1) / kTabLines), kTabLines, 0, st>>>(tab, pl, pu, evy, evz, nky,
                                                                                        nlines, g.nx, nsmall);
   return cudaGetLastError();
@@ -689,12 +691,12 @@ inline bool pois_x_narrow(long nlines) { return nlines < 148L * 4 * 128; }
 
 template <class R>
 cudaError_t pois_x(cudaStream_t st, R *spec, double *aux, const double *pl, const double *pu, const double *evy,
-                   const double *evz, Grid3 g, bool gauge0, unsigned long long *small_pivots,
+                   const double *evz, Grid3 g, bool whole_lines, bool gauge0, unsigned long long *small_pivots,
                    const unsigned long long *nsmall) {
   using namespace svof_cline;
   const long nlines = (long)(g.ny / 2 + 1) * g.nz;
   const int gz = gauge0 ? 1 : 0;
-  if (pois_x_whole_lines(nlines, g.nx)) {
+  if (whole_lines) {
     return cline_by_lpb(cline_lpb(nlines, g.nx, sizeof(R)), [&](auto c) {
       constexpr int LPB = decltype(c)::value;
       k_cline_solve<R, LPB><<<(unsigned)((nlines + LPB - 1) / LPB), 32, cline_smem(LPB, g.nx, sizeof(R)), st>>>(
@@ -771,12 +773,13 @@ cudaError_t pois_resid(cudaStream_t st, const double *b, const double *psi, doub
 }
 
 #define SVOF3_POISSON_INST(R)                                                                                    \
-  template cudaError_t pois_prepare<R>(int, int, int);                                                           \
+  template cudaError_t pois_prepare<R>(int, int, int, bool);                                                     \
   template cudaError_t pois_fwd_y<R>(cudaStream_t, const double *, const double *, const double *, double *, R *, \
                                      const R *, const double *, double, int, Grid3);                            \
   template cudaError_t pois_z<R>(cudaStream_t, R *, const R *, int, Grid3);                                      \
   template cudaError_t pois_x<R>(cudaStream_t, R *, double *, const double *, const double *, const double *,   \
-                                 const double *, Grid3, bool, unsigned long long *, const unsigned long long *); \
+                                 const double *, Grid3, bool, bool, unsigned long long *,                       \
+                                 const unsigned long long *);                                                   \
   template cudaError_t pois_inv_y<R>(cudaStream_t, const R *, double *, const R *, int, Grid3, bool);          \
   template cudaError_t pois_fwd_y_array<R>(cudaStream_t, const double *, R *, const R *, int, Grid3);
 SVOF3_POISSON_INST(double)

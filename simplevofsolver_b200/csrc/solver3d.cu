@@ -13,6 +13,7 @@
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <functional>
 #include <map>
@@ -133,6 +134,10 @@ struct svof3d_solver {
   DevBuf twf_y32, twb_y32, twf_z32, twb_z32;  // FP32 twiddles (SVOF3_MIXED_DC)
   // predictor forward-sweep scratch
   DevBuf fw;
+  // the Poisson solve's x lines whole on chip (where the grid is not too large
+  // for that).  SVOF3_POISSON_LINES = 0 / 1 in the environment of a solver's
+  // creation forces either form, as far as a line fits (tests compare them).
+  bool pois_whole = false;
   // time step
   double *d_dt = nullptr;
   unsigned long long *d_minbits = nullptr;
@@ -359,7 +364,7 @@ int launch_potential_dc(svof3d_solver *s, int rk, const Marker &mark) {
     if (m(SVOF3_K_POISSON_FWD)) return 1;
     CK(pois_z<float>(s->stream, sp, s->twf_z32.as<float>(), s->log2nz, g));
     if (m(SVOF3_K_POISSON_Z)) return 1;
-    CK(pois_x<float>(s->stream, sp, s->xaux.p, s->pl.p, s->pu.p, s->evy.p, s->evz.p, g, true, s->d_health + 1,
+    CK(pois_x<float>(s->stream, sp, s->xaux.p, s->pl.p, s->pu.p, s->evy.p, s->evz.p, g, s->pois_whole, true, s->d_health + 1,
                      s->d_health + 2));
     if (m(SVOF3_K_POISSON_SOLVE)) return 1;
     CK(pois_z<float>(s->stream, sp, s->twb_z32.as<float>(), s->log2nz, g));
@@ -391,7 +396,7 @@ int launch_potential(svof3d_solver *s, int rk, const Marker &mark = Marker()) {
   if (m(SVOF3_K_POISSON_FWD)) return 1;
   CK(pois_z<double>(s->stream, s->spec.p, s->twf_z.p, s->log2nz, g));
   if (m(SVOF3_K_POISSON_Z)) return 1;
-  CK(pois_x<double>(s->stream, s->spec.p, s->xaux.p, s->pl.p, s->pu.p, s->evy.p, s->evz.p, g, false,
+  CK(pois_x<double>(s->stream, s->spec.p, s->xaux.p, s->pl.p, s->pu.p, s->evy.p, s->evz.p, g, s->pois_whole, false,
                     s->d_health + 1, s->d_health + 2));
   if (m(SVOF3_K_POISSON_SOLVE)) return 1;
   CK(pois_z<double>(s->stream, s->spec.p, s->twb_z.p, s->log2nz, g));
@@ -740,8 +745,11 @@ int svof3d_create(const svof3d_params_t *prm, const double *xf, const double *xc
       dalloc(s->fw, 4 * nx * ny * nz, es))
     return bail();
   {
-    const cudaError_t pe =
-        s->dc ? pois_prepare<float>(s->nx, s->log2ny, s->log2nz) : pois_prepare<double>(s->nx, s->log2ny, s->log2nz);
+    const long nlines = (long)nky * s->nz;
+    s->pois_whole = pois_x_whole_lines(nlines, s->nx);
+    if (const char *e = std::getenv("SVOF3_POISSON_LINES")) s->pois_whole = 0 != std::atoi(e) && pois_x_fits(nlines, s->nx);
+    const cudaError_t pe = s->dc ? pois_prepare<float>(s->nx, s->log2ny, s->log2nz, s->pois_whole)
+                                 : pois_prepare<double>(s->nx, s->log2ny, s->log2nz, s->pois_whole);
     if (cudaSuccess != pe || cudaSuccess != predict_prepare(s->nx, (long)s->ny * s->nz) || cudaSuccess != interface_prepare())
       return fail("cudaFuncSetAttribute(Poisson): %s", cudaGetErrorString(cudaGetLastError())), bail();
     const size_t coef_smem = sizeof(double) * 6 * nx;
@@ -759,8 +767,8 @@ int svof3d_create(const svof3d_params_t *prm, const double *xf, const double *xc
       cudaSuccess != cudaMemset(s->d_health, 0, 3 * sizeof(unsigned long long)))
     return fail("cudaMalloc status"), bail();
   if (cudaSuccess != cudaDeviceSynchronize() ||
-      cudaSuccess != pois_x_table(s->stream, s->xaux.p, s->pl.p, s->pu.p, s->evy.p, s->evz.p, s->grid(),
-                                  s->d_health + 2))
+      (s->pois_whole && cudaSuccess != pois_x_table(s->stream, s->xaux.p, s->pl.p, s->pu.p, s->evy.p, s->evz.p,
+                                                    s->grid(), s->d_health + 2)))
     return fail("svof3d_create: Poisson pivots: %s", cudaGetErrorString(cudaGetLastError())), bail();
   {
     const double one = 1.;
@@ -1327,7 +1335,7 @@ int adj3_ensure(svof3d_solver *s) {
   if (!bad && a->f32) bad = dalloc(a->zx, nf) || dalloc(a->zy, nc) || dalloc(a->zz, nc);
   if (!bad && s->mixed)
     bad = dalloc(a->nrm64, 4 * nx * (ny + 2) * (nz + 2)) || dalloc(a->curv64, ncc) ||
-          (s->dc && cudaSuccess != pois_prepare<double>(s->nx, s->log2ny, s->log2nz));
+          (s->dc && cudaSuccess != pois_prepare<double>(s->nx, s->log2ny, s->log2nz, s->pois_whole));
   a->xs_smem = adj_xsolve_smem((int)nx);
   // (FP32 intermediates take the floor too: the exact transposes carry values
   // up to ~1e9 at corners of round-off gradients, beyond FP32's resolution)
@@ -1401,7 +1409,7 @@ int adj3_potential(svof3d_solver *s, int rk, double dt) {
   CK_LAUNCH();
   CK(pois_fwd_y_array<double>(s->stream, a->b.p, s->spec.p, s->twf_y.p, s->log2ny, g));
   CK(pois_z<double>(s->stream, s->spec.p, s->twf_z.p, s->log2nz, g));
-  CK(pois_x<double>(s->stream, s->spec.p, s->xaux.p, s->pl.p, s->pu.p, s->evy.p, s->evz.p, g));
+  CK(pois_x<double>(s->stream, s->spec.p, s->xaux.p, s->pl.p, s->pu.p, s->evy.p, s->evz.p, g, s->pois_whole));
   CK(pois_z<double>(s->stream, s->spec.p, s->twb_z.p, s->log2nz, g));
   CK(pois_inv_y<double>(s->stream, s->spec.p, a->psis.p, s->twb_y.p, s->log2ny, g, false));
   const double pre_p = 1. / (gam * dt) / (1. * s->ny * s->nz);

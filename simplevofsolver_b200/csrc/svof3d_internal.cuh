@@ -161,15 +161,19 @@ __global__ void k3_tdm_coef(const double *__restrict__ lap_ux, const double *__r
 // solve is FP64.  The transforms are compiled for each length 2^1 .. 2^11
 // (log2n outside that range is an invalid value).
 template <class R>
-cudaError_t pois_prepare(int nx, int log2ny, int log2nz);
+cudaError_t pois_prepare(int nx, int log2ny, int log2nz, bool whole_lines);
 // (b: scratch of nx ny nz doubles for the right-hand side)
 template <class R>
 cudaError_t pois_fwd_y(cudaStream_t st, const double *ux, const double *uy, const double *uz, double *b, R *spec,
                        const R *tw, const double *dtp, double gam, int log2n, Grid3 g);
 template <class R>
 cudaError_t pois_z(cudaStream_t st, R *spec, const R *tw, int log2n, Grid3 g);
-// the x line solves' pivots into aux (nx per line, cline_solve.cuh) where
-// pois_x takes whole lines, and the number of lines other than ky = kz = 0
+// whether a line of nx points fits k_cline_solve at all, and whether pois_x
+// takes whole lines of its own accord
+bool pois_x_fits(long nlines, int nx);
+bool pois_x_whole_lines(long nlines, int nx);
+// for whole lines: the x solves' pivots into aux (nx per line,
+// cline_solve.cuh), and the number of lines other than ky = kz = 0
 // that meet one of magnitude at most DBL_EPSILON (+= *nsmall)
 cudaError_t pois_x_table(cudaStream_t st, double *aux, const double *pl, const double *pu, const double *evy,
                          const double *evz, Grid3 g, unsigned long long *nsmall);
@@ -179,8 +183,8 @@ cudaError_t pois_x_table(cudaStream_t st, double *aux, const double *pl, const d
 // magnitude at most DBL_EPSILON)
 template <class R>
 cudaError_t pois_x(cudaStream_t st, R *spec, double *aux, const double *pl, const double *pu, const double *evy,
-                   const double *evz, Grid3 g, bool gauge0 = false, unsigned long long *small_pivots = nullptr,
-                   const unsigned long long *nsmall = nullptr);
+                   const double *evz, Grid3 g, bool whole_lines, bool gauge0 = false,
+                   unsigned long long *small_pivots = nullptr, const unsigned long long *nsmall = nullptr);
 // acc: psi += the result (the correction pass), the walls' halo images kept
 template <class R>
 cudaError_t pois_inv_y(cudaStream_t st, const R *spec, double *psi, const R *tw, int log2n, Grid3 g,
