@@ -807,7 +807,7 @@ cudaError_t by_xl_shape(int nx, F f) {
 }
 
 template <class R>
-cudaError_t predict_launch(cudaStream_t st, const Predict3Args<R> &a) {
+cudaError_t predict_launch(cudaStream_t st, const Predict3Args<R> &a, bool whole_lines) {
   const Grid3 &g = a.g;
   const int planes = march_planes_even((long)((g.nx + RX - 1) / RX) * ((g.ny + RY - 1) / RY), g.nz, 64, 2, 3);
   dim3 gr((g.nx + RX - 1) / RX, (g.ny + RY - 1) / RY, (g.nz + planes - 1) / planes);
@@ -818,7 +818,7 @@ cudaError_t predict_launch(cudaStream_t st, const Predict3Args<R> &a) {
   const long nlines = (long)g.ny * g.nz;
   return by_xl_shape(g.nx, [&](auto shape) {
     using S = decltype(shape);
-    const int nw = xlines_warps<R, S>(g.nx, nlines);
+    const int nw = whole_lines ? xlines_warps<R, S>(g.nx, nlines) : 0;
     if (nw > 0) {
       const unsigned blocks = (unsigned)std::min<long>(148, (4 * nlines * S::XLP / 32 + nw - 1) / nw);
       k3_xlines<R, S><<<blocks, 32 * nw, xl_table_bytes<R>(g.nx) + nw * xl_warp_bytes<R, S>(g.nx), st>>>(a);
@@ -843,11 +843,11 @@ cudaError_t predict_prepare_t(int nx, long nlines) {
   return raise_smem_limit(k3_rhs<R, true>, kRhsSmem<R>);
 }
 #if SVOF3_WITH_F64
-template cudaError_t predict_launch<double>(cudaStream_t, const Predict3Args<double> &);
+template cudaError_t predict_launch<double>(cudaStream_t, const Predict3Args<double> &, bool);
 template cudaError_t predict_prepare_t<double>(int, long);
 #endif
 #if SVOF3_WITH_F32
-template cudaError_t predict_launch<float>(cudaStream_t, const Predict3Args<float> &);
+template cudaError_t predict_launch<float>(cudaStream_t, const Predict3Args<float> &, bool);
 template cudaError_t predict_prepare_t<float>(int, long);
 #endif
 

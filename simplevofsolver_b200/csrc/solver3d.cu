@@ -134,10 +134,11 @@ struct svof3d_solver {
   DevBuf twf_y32, twb_y32, twf_z32, twb_z32;  // FP32 twiddles (SVOF3_MIXED_DC)
   // predictor forward-sweep scratch
   DevBuf fw;
-  // the Poisson solve's x lines whole on chip (where the grid is not too large
-  // for that).  SVOF3_POISSON_LINES = 0 / 1 in the environment of a solver's
-  // creation forces either form, as far as a line fits (tests compare them).
-  bool pois_whole = false;
+  // x line solves on whole lines (the Poisson solve's: where the grid is not
+  // too large for them; the predictor's: where a line fits).  The environment's
+  // SVOF3_POISSON_LINES and SVOF3_PREDICT_LINES = 0 / 1 at a solver's creation
+  // force either form, as far as a line fits (tests compare them).
+  bool pois_whole = false, pred_whole = true;
   // time step
   double *d_dt = nullptr;
   unsigned long long *d_minbits = nullptr;
@@ -313,7 +314,7 @@ int launch_predict_t(svof3d_solver *s, int rk) {
   a.grav_vof = s->grav_vof;
   a.vof_ref = s->vof_ref;
   a.g = s->grid();
-  CK(predict_launch<R>(s->stream, a));
+  CK(predict_launch<R>(s->stream, a, s->pred_whole));
   return 0;
 }
 
@@ -748,6 +749,7 @@ int svof3d_create(const svof3d_params_t *prm, const double *xf, const double *xc
     const long nlines = (long)nky * s->nz;
     s->pois_whole = pois_x_whole_lines(nlines, s->nx);
     if (const char *e = std::getenv("SVOF3_POISSON_LINES")) s->pois_whole = 0 != std::atoi(e) && pois_x_fits(nlines, s->nx);
+    if (const char *e = std::getenv("SVOF3_PREDICT_LINES")) s->pred_whole = 0 != std::atoi(e);
     const cudaError_t pe = s->dc ? pois_prepare<float>(s->nx, s->log2ny, s->log2nz, s->pois_whole)
                                  : pois_prepare<double>(s->nx, s->log2ny, s->log2nz, s->pois_whole);
     if (cudaSuccess != pe || cudaSuccess != predict_prepare(s->nx, (long)s->ny * s->nz) || cudaSuccess != interface_prepare())

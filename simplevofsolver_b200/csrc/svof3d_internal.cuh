@@ -141,8 +141,9 @@ struct Predict3Args {
   double grav_vof, vof_ref;
   Grid3 g;
 };
+// (whole_lines false: k3_xsolve at every line length, else only where k3_xlines does not fit)
 template <class R>
-cudaError_t predict_launch(cudaStream_t st, const Predict3Args<R> &a);
+cudaError_t predict_launch(cudaStream_t st, const Predict3Args<R> &a, bool whole_lines);
 // opt-in shared memory of the predictor's kernels (lines of nx cells; once per device)
 cudaError_t predict_prepare(int nx, long nlines);
 // Thomas coefficients of up to three substeps for the three distinct systems,
