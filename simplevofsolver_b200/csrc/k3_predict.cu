@@ -12,7 +12,8 @@
 //   k3_xlines  the x lines (ny nz of them): a few whole lines a warp, in
 //              segments over its lanes, and the updated fields with their halo
 //              images and walls
-//   k3_xsolve  the same for lines too long for that: a block owns
+//   k3_xsolve  the same for lines too long for that, and for grids of many
+//              lines where the implicit x is strong: a block owns
 //              32 lines, walks them in 32-cell chunks forward and backward
 //              with one line per lane of four sweeping warps, and writes the
 //              updated fields with their halo images and walls
@@ -24,7 +25,9 @@
 // in FP32); R is the storage type of forces, sources and increments.
 #include <cuda_pipeline.h>
 
+#include <algorithm>
 #include <type_traits>
+#include <vector>
 
 #include "svof3d_internal.cuh"
 #include "smem_limit.cuh"
@@ -52,8 +55,9 @@ namespace svof3 {
 #if SVOF3_WITH_F64
 __global__ void k3_tdm_coef(const double *__restrict__ lap_ux, const double *__restrict__ lap_cc,
                             const double *__restrict__ dtp, Gam3 gams, double m_dif, double t_dif, int nx,
-                            double *__restrict__ coef_all) {
-  // block b: the table of gamma = gams.g[b] at coef_all + 9 nx b
+                            double *__restrict__ coef_all, PredictRounds rounds, int *__restrict__ stream_lines) {
+  // block b: the table of gamma = gams.g[b] at coef_all + 9 nx b, and whether
+  // its lines are streamed to stream_lines[b] (where rounds.limit is set)
   const double gam = gams.g[blockIdx.x];
   double *coef = coef_all + (size_t)9 * nx * blockIdx.x;
   extern __shared__ double slap[];  // [2][3 nx]
@@ -64,15 +68,33 @@ __global__ void k3_tdm_coef(const double *__restrict__ lap_ux, const double *__r
   }
   __syncthreads();
   const int f = threadIdx.x >> 5;  // a warp a system
-  if (f >= 3) return;
-  const double *lap = slap + ((0 == f) ? 0 : 3 * nx);
-  const double dif = (2 == f) ? t_dif : m_dif;
-  const int n = (0 == f) ? nx - 1 : nx;
-  double *L = coef + (size_t)(3 * f + 0) * nx;
-  double *R = coef + (size_t)(3 * f + 1) * nx;
-  double *V = coef + (size_t)(3 * f + 2) * nx;
-  const double pf = 0.5 * gam * *dtp * dif;
-  svof_tdm::pivots(lap, pf, n, L, R, V);
+  __shared__ int most[3];
+  if (f < 3) {
+    const double *lap = slap + ((0 == f) ? 0 : 3 * nx);
+    const double dif = (2 == f) ? t_dif : m_dif;
+    const int n = (0 == f) ? nx - 1 : nx;
+    double *L = coef + (size_t)(3 * f + 0) * nx;
+    double *R = coef + (size_t)(3 * f + 1) * nx;
+    double *V = coef + (size_t)(3 * f + 2) * nx;
+    const double pf = 0.5 * gam * *dtp * dif;
+    svof_tdm::pivots(lap, pf, n, L, R, V);
+    if (rounds.limit > 0) {
+      __syncwarp();  // the table is read by other lanes than wrote it
+      // lanes s and 16 + s: the boundaries s, forward and backward
+      const int s = threadIdx.x & 15;
+      const bool back = 0 != (threadIdx.x & 16);
+      int r = 0;
+      if (s > 0 && s < rounds.lanes)
+        r = svof_tdm::boundary_rounds(L, R, V, n, rounds.seg, s, rounds.warm, rounds.eps, back,
+                                      rounds.limit);
+      const int fwd = __reduce_max_sync(0xffffffffu, back ? 0 : r), bwd = __reduce_max_sync(0xffffffffu, back ? r : 0);
+      if (0 == (threadIdx.x & 31)) most[f] = fwd + bwd;
+    }
+  }
+  if (rounds.limit > 0) {
+    __syncthreads();
+    if (0 == threadIdx.x) stream_lines[blockIdx.x] = max(most[0], max(most[1], most[2])) >= rounds.limit;
+  }
 }
 #endif
 
@@ -483,6 +505,7 @@ using SweepT = typename std::conditional<4 == sizeof(R), float, double>::type;
 
 template <class R>
 __global__ void __launch_bounds__(256) k3_xsolve(Predict3Args<R> a) {
+  if (a.stream_lines && 0 == *a.stream_lines) return;
   constexpr int NB = kXsBufs<R>;
   using T = SweepT<R>;
   __shared__ R sd[NB][4][PL][PC + 1];  // the four fields' values of one tile
@@ -724,6 +747,7 @@ __device__ __forceinline__ void prefetch_l2(const void *p, long bytes, int lane)
 
 template <class R, class S>
 __global__ void __launch_bounds__(S::MAXW * 32) k3_xlines(Predict3Args<R> a) {
+  if (a.stream_lines && 0 != *a.stream_lines) return;
   using T = SweepT<R>;
   constexpr int XLP = S::XLP, XLB = 32 / XLP;
   extern __shared__ double smd[];
@@ -822,11 +846,59 @@ cudaError_t predict_launch(cudaStream_t st, const Predict3Args<R> &a, bool whole
     if (nw > 0) {
       const unsigned blocks = (unsigned)std::min<long>(148, (4 * nlines * S::XLP / 32 + nw - 1) / nw);
       k3_xlines<R, S><<<blocks, 32 * nw, xl_table_bytes<R>(g.nx) + nw * xl_warp_bytes<R, S>(g.nx), st>>>(a);
-    } else {
-      k3_xsolve<R><<<(unsigned)((nlines + PL - 1) / PL), 256, 0, st>>>(a);
+      const cudaError_t le = cudaGetLastError();
+      if (cudaSuccess != le || !a.stream_lines) return le;
     }
+    k3_xsolve<R><<<(unsigned)((nlines + PL - 1) / PL), 256, 0, st>>>(a);
     return cudaGetLastError();
   });
+}
+
+// Where the implicit x is strong (|V| near 1: wall-clustered or flat cells near
+// the diffusive limit), segments meet late and are run again, round after
+// round; the chain of k3_xsolve does not care, but it needs many lines to fill
+// the chip.  From 16384 lines on it is the faster one from 3 rounds a line
+// (both directions) in FP64 and 5 in FP32, 2 and 3 with segments of 8 lanes;
+// from 8192 lines twice that, below never.  us a step, k3_xlines / k3_xsolve,
+// by rounds: FP64 512 x 16384 lines 0: 3720 / 4210, 2: 4098 / 4215, 4: 4309 /
+// 4206, 6: 4854 / 4238; 1000 x 16384 2: 8548 / 8609, 4: 9392 / 8594, 8: 10590 /
+// 8644; 256 x 16384 1: 2099 / 2132, 2: 2162 / 2134; 512 x 8192 5: 2456 / 2508,
+// 7: 2530 / 2507; 512 x 4096 8: 1461 / 1585; FP32 512 x 16384 4: 3738 / 3782,
+// 5: 3835 / 3773; 320 x 16384 2: 2448 / 2403, 3: 2529 / 2404.
+template <class R>
+PredictRounds predict_rounds(const double *lap_ux, const double *lap_cc, int nx, long nlines, double pf_max) {
+  PredictRounds p{};
+  by_xl_shape(nx, [&](auto shape) {
+    using S = decltype(shape);
+    if (nlines < 8192 || xlines_warps<R, S>(nx, nlines) < 1) return cudaSuccess;
+    constexpr int few = 16 == S::XLP ? (8 == sizeof(R) ? 3 : 5) : (8 == sizeof(R) ? 2 : 3);
+    p = PredictRounds{S::XLP, xl_seg<S>(nx), kXlWarm<R>, nlines < 16384 ? 2 * few : few,
+                      8 == sizeof(R) ? 0x1p-53 : 0x1p-24};
+    return cudaSuccess;
+  });
+  if (0 == p.limit) return p;
+  int most = 0;
+  for (const double *lap : {lap_ux, lap_cc}) {
+    const int n = lap == lap_ux ? nx - 1 : nx;
+    std::vector<double> L(n), r(n), V(n);
+    for (int i = 0; i < n; i++) {
+      L[i] = -pf_max * lap[3 * i];
+      const double c = 1. - pf_max * lap[3 * i + 1];
+      r[i] = 1. / (i > 0 ? c - L[i] * V[i - 1] : c);
+      V[i] = r[i] * (-pf_max * lap[3 * i + 2]);
+    }
+    int fwd = 0, bwd = 0;
+    for (int s = 1; s < p.lanes; s++) {
+      auto rounds = [&](bool backward) {
+        return svof_tdm::boundary_rounds(L.data(), r.data(), V.data(), n, p.seg, s, p.warm, p.eps, backward, p.limit);
+      };
+      fwd = std::max(fwd, rounds(false));
+      bwd = std::max(bwd, rounds(true));
+    }
+    most = std::max(most, fwd + bwd);
+  }
+  if (most < p.limit) p.limit = 0;
+  return p;
 }
 
 template <class R>
@@ -843,10 +915,12 @@ cudaError_t predict_prepare_t(int nx, long nlines) {
   return raise_smem_limit(k3_rhs<R, true>, kRhsSmem<R>);
 }
 #if SVOF3_WITH_F64
+template PredictRounds predict_rounds<double>(const double *, const double *, int, long, double);
 template cudaError_t predict_launch<double>(cudaStream_t, const Predict3Args<double> &, bool);
 template cudaError_t predict_prepare_t<double>(int, long);
 #endif
 #if SVOF3_WITH_F32
+template PredictRounds predict_rounds<float>(const double *, const double *, int, long, double);
 template cudaError_t predict_launch<float>(cudaStream_t, const Predict3Args<float> &, bool);
 template cudaError_t predict_prepare_t<float>(int, long);
 #endif

@@ -135,10 +135,14 @@ struct svof3d_solver {
   // predictor forward-sweep scratch
   DevBuf fw;
   // x line solves on whole lines (the Poisson solve's: where the grid is not
-  // too large for them; the predictor's: where a line fits).  The environment's
-  // SVOF3_POISSON_LINES and SVOF3_PREDICT_LINES = 0 / 1 at a solver's creation
-  // force either form, as far as a line fits (tests compare them).
+  // too large for them; the predictor's: where a line fits and its segments
+  // need not be run again too often, which pred_rounds has judged each substep
+  // into stream_lines where it can be).  The environment's SVOF3_POISSON_LINES
+  // and SVOF3_PREDICT_LINES = 0 / 1 at a solver's creation force either form, as
+  // far as a line fits (tests compare them).
   bool pois_whole = false, pred_whole = true;
+  PredictRounds pred_rounds{};
+  DevBuf stream_lines;  // an int a substep
   // time step
   double *d_dt = nullptr;
   unsigned long long *d_minbits = nullptr;
@@ -313,6 +317,7 @@ int launch_predict_t(svof3d_solver *s, int rk) {
   a.vof = s->vof[s->cur_v].p;  // after this substep's advection
   a.grav_vof = s->grav_vof;
   a.vof_ref = s->vof_ref;
+  a.stream_lines = s->pred_rounds.limit > 0 ? s->stream_lines.as<int>() + rk : nullptr;
   a.g = s->grid();
   CK(predict_launch<R>(s->stream, a, s->pred_whole));
   return 0;
@@ -325,7 +330,7 @@ int launch_coef(svof3d_solver *s, int rk, cudaStream_t st) {
   for (int q = 0; q < 3; q++) g.g[q] = (rk < 0) ? RK_A[q] + RK_B[q] : RK_A[rk] + RK_B[rk];
   k3_tdm_coef<<<rk < 0 ? 3 : 1, 256, sizeof(double) * 6 * s->nx, st>>>(
       s->lap_ux.p, s->lap_cc.p, s->d_dt, g, s->prm.m_dif, s->prm.t_dif, s->nx,
-      s->coef.p + (size_t)9 * s->nx * std::max(rk, 0));
+      s->coef.p + (size_t)9 * s->nx * std::max(rk, 0), s->pred_rounds, s->stream_lines.as<int>() + std::max(rk, 0));
   CK_LAUNCH();
   return 0;
 }
@@ -604,6 +609,19 @@ int build_tables(svof3d_solver *s, const double *xf, const double *xc) {
   s->lims[1] = cd / s->prm.m_dif * 0.5 / ndims * std::pow(s->dz, 2.);
   s->lims[2] = cd / s->prm.t_dif * 0.5 / ndims * std::pow(s->dy, 2.);
   s->lims[3] = cd / s->prm.t_dif * 0.5 / ndims * std::pow(s->dz, 2.);
+  {
+    double dt = s->prm.coef_dt_adv;  // the largest that k3_dt_final gives
+    for (double lim : s->lims) dt = std::min(dt, lim);
+    double gam = 0.;
+    for (int rk = 0; rk < 3; rk++) gam = std::max(gam, RK_A[rk] + RK_B[rk]);
+    const double pf = 0.5 * gam * dt * std::max(s->prm.m_dif, s->prm.t_dif);
+    const long nlines = (long)ny * nz;
+    const char *e = std::getenv("SVOF3_PREDICT_LINES");
+    if (e) s->pred_whole = 0 != std::atoi(e);
+    else s->pred_rounds = s->mixed ? predict_rounds<float>(lux.data(), lcc.data(), nx, nlines, pf)
+                                   : predict_rounds<double>(lux.data(), lcc.data(), nx, nlines, pf);
+    if (dalloc(s->stream_lines, 3)) return 1;
+  }
   s->log2ny = ilog2_exact(ny);
   s->log2nz = ilog2_exact(nz);
   if (s->log2ny < 1 || s->log2nz < 1) return fail("svof3d_create: ny and nz must be powers of two (got %d, %d)", ny, nz);
@@ -667,7 +685,7 @@ int svof3d_destroy(svof3d_solver_t *s) {
     dfree(s->sux[k]); dfree(s->suy[k]); dfree(s->suz[k]); dfree(s->st[k]); dfree(s->svof[k]);
   }
   DevBuf *bufs[] = {&s->p, &s->psi, &s->curv, &s->normal, &s->ifrcx, &s->ifrcy, &s->ifrcz, &s->dxf, &s->dxc,
-                    &s->lap_ux, &s->lap_cc, &s->coef, &s->spec, &s->xaux, &s->twf_y, &s->twb_y, &s->twf_z,
+                    &s->lap_ux, &s->lap_cc, &s->coef, &s->stream_lines, &s->spec, &s->xaux, &s->twf_y, &s->twb_y, &s->twf_z,
                     &s->twb_z, &s->pl, &s->pu, &s->evy, &s->evz, &s->fw, &s->diag, &s->stat_part,
                     &s->twf_y32, &s->twb_y32, &s->twf_z32, &s->twb_z32};
   for (DevBuf *b : bufs) dfree(*b);
@@ -749,7 +767,6 @@ int svof3d_create(const svof3d_params_t *prm, const double *xf, const double *xc
     const long nlines = (long)nky * s->nz;
     s->pois_whole = pois_x_whole_lines(nlines, s->nx);
     if (const char *e = std::getenv("SVOF3_POISSON_LINES")) s->pois_whole = 0 != std::atoi(e) && pois_x_fits(nlines, s->nx);
-    if (const char *e = std::getenv("SVOF3_PREDICT_LINES")) s->pred_whole = 0 != std::atoi(e);
     const cudaError_t pe = s->dc ? pois_prepare<float>(s->nx, s->log2ny, s->log2nz, s->pois_whole)
                                  : pois_prepare<double>(s->nx, s->log2ny, s->log2nz, s->pois_whole);
     if (cudaSuccess != pe || cudaSuccess != predict_prepare(s->nx, (long)s->ny * s->nz) || cudaSuccess != interface_prepare())

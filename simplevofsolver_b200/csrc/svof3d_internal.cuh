@@ -139,11 +139,26 @@ struct Predict3Args {
   // vof_ref), vof the field after this substep's advection (storage layout)
   const double *vof;
   double grav_vof, vof_ref;
+  // when given: 0 where this substep's lines go to k3_xlines, else to k3_xsolve
+  // (both are launched); when not, predict_launch's whole_lines decides
+  const int *stream_lines;
   Grid3 g;
 };
 // (whole_lines false: k3_xsolve at every line length, else only where k3_xlines does not fit)
 template <class R>
 cudaError_t predict_launch(cudaStream_t st, const Predict3Args<R> &a, bool whole_lines);
+// When the x lines' segments (k3_xlines) have to be run again so often that
+// k3_xsolve is faster: the segments' shape and the rounds a substep from which
+// on that is so (0: never).  Made for a grid by predict_rounds, judged by
+// k3_tdm_coef with the step's coefficients.
+struct PredictRounds {
+  int lanes, seg, warm, limit;
+  double eps;
+};
+// (lap_ux, lap_cc: host copies; pf_max: the largest prefactor 0.5 gamma dt nu
+// of a step.  Limit 0 where no step within it gets that far)
+template <class R>
+PredictRounds predict_rounds(const double *lap_ux, const double *lap_cc, int nx, long nlines, double pf_max);
 // opt-in shared memory of the predictor's kernels (lines of nx cells; once per device)
 cudaError_t predict_prepare(int nx, long nlines);
 // Thomas coefficients of up to three substeps for the three distinct systems,
@@ -153,7 +168,7 @@ struct Gam3 {
 };
 __global__ void k3_tdm_coef(const double *__restrict__ lap_ux, const double *__restrict__ lap_cc,
                             const double *__restrict__ dtp, Gam3 gams, double m_dif, double t_dif, int nx,
-                            double *__restrict__ coef_all);
+                            double *__restrict__ coef_all, PredictRounds rounds, int *__restrict__ stream_lines);
 
 // Poisson: spectral array S[kz][ky][i] (complex, i fastest)
 // Poisson stages (k3_poisson.cu), templates on R, the type of the spectrum,

@@ -83,6 +83,39 @@ __device__ __forceinline__ void pivots(const double *lap, double pf, int n, doub
   }
 }
 
+// How often a line's segments have to be run again, from the table alone: a
+// difference ahead of a segment shrinks by |R_i L_i| a row forward and by |V_i|
+// a row backward; the rows it takes to fall below eps, beyond the `warm` ahead
+// of each segment, run through one more segment a round.  The rounds of the
+// boundary below row a = 1 + s seg (n rows; forward as far as row 1, backward
+// as far as row n - 2, where the true value is known), at most `limit`.
+__host__ __device__ inline int boundary_rounds(const double *L, const double *R, const double *V, int n, int seg, int s,
+                                               int warm, double eps, bool backward, int limit) {
+  constexpr int B = 8;  // rows whose loads are in flight together
+  const int a = 1 + s * seg;
+  if (a >= n - 1) return 0;
+  const int have = backward ? n - 1 - a : a - 1;
+  const int most = warm + (limit - 1) * seg + 1, last = have < most ? have : most;
+  double p = 1.;
+  int rows = 0;
+  while (rows < last && p > eps) {
+    double c[B];
+#pragma unroll
+    for (int k = 0; k < B; k++) {
+      const int q = rows + k < last ? rows + k : last - 1;
+      c[k] = backward ? V[a + q] : R[a - 1 - q] * L[a - 1 - q];
+    }
+#pragma unroll
+    for (int k = 0; k < B; k++) {
+      if (rows < last && p > eps) {
+        p *= fabs(c[k]);
+        rows++;
+      }
+    }
+  }
+  return rows <= warm ? 0 : (rows - warm + seg - 1) / seg;
+}
+
 __device__ __forceinline__ bool same_bits(double a, double b) {
   return __double_as_longlong(a) == __double_as_longlong(b);
 }
