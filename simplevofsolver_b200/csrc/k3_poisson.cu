@@ -606,20 +606,30 @@ cudaError_t line_attrs(K kernel, int smem) {
 }
 }  // namespace
 
-// whole lines in shared memory where the chip takes all of them in at most
-// 12 rounds: beyond that the chip holds too few lines at a time (their
-// latency, not the bytes, is then what counts) and k3_pois_x streams near the
-// copy rate.  us a launch, whole lines against k3_pois_x: 61 x 64 x 32 10 /
-// 28, 128^3 18 / 53, 256^3 (6 rounds) 116 / 153, 512^3 (44) 1300 / 955.
+// Whole lines in shared memory where the chip takes all of them in few rounds:
+// beyond that the chip holds too few lines at a time (their latency, not the
+// bytes, is then what counts) and k3_pois_x streams near the copy rate.  FP64
+// up to 12 rounds, 8 where a warp has one or two lines (long ones), 2 where
+// lines are so short that the streaming kernel's chunk holds them whole; FP32
+// storage up to 8, fewer below 128 cells.  us a launch, whole lines against
+// k3_pois_x: 61 x 64 x 32 10 / 28, 128^3 18 / 53, 256^3 (6 rounds) 116 / 153,
+// 512^3 (44) 1300 / 955.  us a call of the whole Poisson solve, FP64: 700 x
+// 16512 lines (7 rounds) 1072 / 1100, 1500 x 8320 (7) 1404 / 1468, 2000 x 8320
+// (9.4) 1926 / 1842, 512 x 33024 (10.1) 1413 / 1320, 256 x 65792 (11.1) 1350 /
+// 1373, 16 x 33024 (1.6) 103 / 103, 16 x 65792 (3.3) 172 / 166; FP32 storage: 128
+// x 65792 (7) 1047 / 1039, 256 x 65792 (11.1) 2047 / 2025, 64 x 33024 (2.5) 319 /
+// 331, 64 x 65792 (5) 584 / 578, 32 x 33024 (1.9) 198 / 202, 32 x 65792 (3.7) 367
+// / 357, 16 x 16512 (0.8) 119 / 123, 16 x 33024 166 / 159.
 static size_t pois_x_block_bytes(long nlines, int nx) {
   return svof_cline::cline_smem(svof_cline::cline_lpb(nlines, nx, sizeof(double)), nx, sizeof(double)) + 1024;
 }
 bool pois_x_fits(long nlines, int nx) { return pois_x_block_bytes(nlines, nx) <= 227 * 1024; }
-bool pois_x_whole_lines(long nlines, int nx) {
+bool pois_x_whole_lines(long nlines, int nx, bool fp32) {
   if (!pois_x_fits(nlines, nx)) return false;
   const int lpb = svof_cline::cline_lpb(nlines, nx, sizeof(double));
   const long held = 148L * lpb * std::min<long>(32, 227 * 1024 / pois_x_block_bytes(nlines, nx));
-  return nlines <= 12 * held;
+  const int rounds = fp32 ? std::max(1, std::min(8, nx / 16)) : (nx < 24 ? 2 : (lpb < 4 ? 8 : 12));
+  return nlines <= rounds * held;
 }
 
 template <class R>

@@ -765,7 +765,7 @@ int svof3d_create(const svof3d_params_t *prm, const double *xf, const double *xc
     return bail();
   {
     const long nlines = (long)nky * s->nz;
-    s->pois_whole = pois_x_whole_lines(nlines, s->nx);
+    s->pois_whole = pois_x_whole_lines(nlines, s->nx, s->dc);
     if (const char *e = std::getenv("SVOF3_POISSON_LINES")) s->pois_whole = 0 != std::atoi(e) && pois_x_fits(nlines, s->nx);
     const cudaError_t pe = s->dc ? pois_prepare<float>(s->nx, s->log2ny, s->log2nz, s->pois_whole)
                                  : pois_prepare<double>(s->nx, s->log2ny, s->log2nz, s->pois_whole);

@@ -184,10 +184,10 @@ cudaError_t pois_fwd_y(cudaStream_t st, const double *ux, const double *uy, cons
                        const R *tw, const double *dtp, double gam, int log2n, Grid3 g);
 template <class R>
 cudaError_t pois_z(cudaStream_t st, R *spec, const R *tw, int log2n, Grid3 g);
-// whether a line of nx points fits k_cline_solve at all, and whether pois_x
-// takes whole lines of its own accord
+// whether a line of nx points fits k_cline_solve at all, and whether a solver
+// takes whole lines (fp32: the spectrum's storage)
 bool pois_x_fits(long nlines, int nx);
-bool pois_x_whole_lines(long nlines, int nx);
+bool pois_x_whole_lines(long nlines, int nx, bool fp32);
 // for whole lines: the x solves' pivots into aux (nx per line,
 // cline_solve.cuh), and the number of lines other than ky = kz = 0
 // that meet one of magnitude at most DBL_EPSILON (+= *nsmall)
