@@ -711,7 +711,7 @@ cudaError_t interface_geom(cudaStream_t st, const double *vof, R *normal, R *cur
   cudaError_t e = cudaMemsetAsync(nwork, 0, sizeof(unsigned), st);
   if (cudaSuccess != e) return e;
   const long columns = (long)((g.nx + G3X - 1) / G3X) * ((g.ny + 2 + G3Y - 1) / G3Y);
-  const int planes = march_planes_uneven(columns, g.nz + 2, 32, 7);
+  const int planes = march_planes_uneven(columns, g.nz + 2, 32, 7, 2.);
   dim3 gr((g.nx + G3X - 1) / G3X, (g.ny + 2 + G3Y - 1) / G3Y, (g.nz + 2 + planes - 1) / planes);
   k3_geom<R><<<gr, G3X * G3Y, 0, st>>>(vof, normal, curv, work, nwork, planes, g);
   if (cudaSuccess != (e = cudaGetLastError())) return e;
@@ -731,7 +731,7 @@ template <class R>
 cudaError_t interface_advect(cudaStream_t st, const double *vof, double *vof_new, const double *ux,
                              const double *uy, const double *uz, const R *normal, double *src_a,
                              const double *src_b, const double *dtp, RK rk, int use_b, Grid3 g) {
-  const int planes = march_planes_uneven((long)((g.nx + AX - 1) / AX) * ((g.ny + AY - 1) / AY), g.nz, 32, 4);
+  const int planes = march_planes_uneven((long)((g.nx + AX - 1) / AX) * ((g.ny + AY - 1) / AY), g.nz, 32, 4, 1.2);
   by_depth(planes, [&](auto c) {
     constexpr int AZ = decltype(c)::value;
     dim3 gr((g.nx + AX - 1) / AX, (g.ny + AY - 1) / AY, (g.nz + AZ - 1) / AZ);

@@ -272,12 +272,14 @@ inline int march_planes_even(long columns, int nz, int most, int resident, int l
 
 // Blocks whose cost depends on the interface they hold (k3_geom,
 // k3_vof_advect): work grows as 1 + lead / d, the tail of uneven blocks as
-// d, hence the square root; 1.2 is the ratio of the two.  Vof advection 61 x
+// d, hence the square root of their ratio (1.2 for the advection, 2 for the
+// geometry: against 1.2, 1000 x 64 x 64 75.6 -> 73.5 us a call, 16 x 1024 x 1024
+// 230 -> 223, 900 x 128 x 256 241 -> 236, 256^3 169 -> 171).  Vof advection 61 x
 // 64 x 32 98 -> 12.6 (1 plane; 2: 18.1), 128^3 mixed 86 -> 53.7 (4; 8:
 // 56.8), 256^3 449 -> 423 (8; 19: 445), 512^3 unchanged (32);
 // geometry 34.4 -> 9.2, 47.9 -> 27.1, 165 -> 151, unchanged.
-inline int march_planes_uneven(long columns, int nz, int most, int resident) {
-  const double d = std::sqrt(1.2 * (double)columns * nz / (148. * resident));
+inline int march_planes_uneven(long columns, int nz, int most, int resident, double ratio) {
+  const double d = std::sqrt(ratio * (double)columns * nz / (148. * resident));
   return std::max(1, std::min({most, nz, (int)(d + 0.5)}));
 }
 
