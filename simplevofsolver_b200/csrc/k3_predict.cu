@@ -915,6 +915,13 @@ cudaError_t predict_prepare_t(int nx, long nlines) {
   return raise_smem_limit(k3_rhs<R, true>, kRhsSmem<R>);
 }
 #if SVOF3_WITH_F64
+// Lines of up to two chunks of k3_xsolve, when there are many: a segment's rows
+// ahead are then most of the line, done over by every lane.  us a call,
+// k3_xlines / k3_xsolve: FP64 16 x 4096 lines 48 / 43, 16 x 2^20 2842 / 1762, 32
+// x 65536 256 / 178, 64 x 65536 378 / 332, 80 x 65536 faster by k3_xlines; mixed
+// 64 x 4096 56 / 56, 64 x 65536 291 / 280; with 1024 lines k3_xlines at any
+// length.
+bool predict_whole_lines(int nx, long nlines) { return nx > 64 || nlines < 4096; }
 template PredictRounds predict_rounds<double>(const double *, const double *, int, long, double);
 template cudaError_t predict_launch<double>(cudaStream_t, const Predict3Args<double> &, bool);
 template cudaError_t predict_prepare_t<double>(int, long);

@@ -617,8 +617,9 @@ int build_tables(svof3d_solver *s, const double *xf, const double *xc) {
     const double pf = 0.5 * gam * dt * std::max(s->prm.m_dif, s->prm.t_dif);
     const long nlines = (long)ny * nz;
     const char *e = std::getenv("SVOF3_PREDICT_LINES");
-    if (e) s->pred_whole = 0 != std::atoi(e);
-    else s->pred_rounds = s->mixed ? predict_rounds<float>(lux.data(), lcc.data(), nx, nlines, pf)
+    s->pred_whole = e ? 0 != std::atoi(e) : predict_whole_lines(nx, nlines);
+    if (!e && s->pred_whole)
+      s->pred_rounds = s->mixed ? predict_rounds<float>(lux.data(), lcc.data(), nx, nlines, pf)
                                    : predict_rounds<double>(lux.data(), lcc.data(), nx, nlines, pf);
     if (dalloc(s->stream_lines, 3)) return 1;
   }

@@ -144,7 +144,9 @@ struct Predict3Args {
   const int *stream_lines;
   Grid3 g;
 };
-// (whole_lines false: k3_xsolve at every line length, else only where k3_xlines does not fit)
+// (whole_lines false: k3_xsolve at every line length, else only where k3_xlines does not fit;
+// predict_whole_lines: which a grid takes)
+bool predict_whole_lines(int nx, long nlines);
 template <class R>
 cudaError_t predict_launch(cudaStream_t st, const Predict3Args<R> &a, bool whole_lines);
 // When the x lines' segments (k3_xlines) have to be run again so often that
