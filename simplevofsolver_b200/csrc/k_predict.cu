@@ -212,8 +212,15 @@ __global__ void __launch_bounds__(256, 3) k_predict(PredictArgs a) {
   __syncthreads();
 
   // ---------------- phase 2: Thomas sweeps (gtsv, src/tdm.c:17-50) with the
-  // coefficients of k_tdm_coef, a warp a line
-  for (int w = tid >> 5; w < 3 * nrows; w += blockDim.x >> 5) {
+  // coefficients of k_tdm_coef, a warp a line, or a thread a line where lines
+  // are short
+  if (a.thread_lines) {
+    if (tid < 3 * nrows) {
+      const int f = tid / nrows, jj = tid - f * nrows;
+      svof_tdm::line_solve_thread(sc + (3 * f + 0) * ld, sc + (3 * f + 1) * ld, sc + (3 * f + 2) * ld,
+                                  (0 == f) ? nx - 1 : nx, sd + (f * R + jj) * ld);
+    }
+  } else for (int w = tid >> 5; w < 3 * nrows; w += blockDim.x >> 5) {
     const int f = w / nrows, jj = w - f * nrows;
     svof_tdm::line_solve(sc + (3 * f + 0) * ld, sc + (3 * f + 1) * ld, sc + (3 * f + 2) * ld, (0 == f) ? nx - 1 : nx,
                          sd + (f * R + jj) * ld, sq + (f * R + jj) * ld);

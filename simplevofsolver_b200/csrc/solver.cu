@@ -238,6 +238,7 @@ int launch_predict(svof_solver *s, int rk, bool with_coef) {
   a.grav_vof = s->grav_vof;
   a.vof_ref = s->vof_ref;
   a.rows_per_block = s->pred_rows;
+  a.thread_lines = s->pred_thread_lines;
   a.g = s->grid();
   if (s->pred_lines) {
     const dim3 tiles((s->nx + 31) / 32, (s->ny + 31) / 32);
@@ -628,11 +629,15 @@ int engine_create(const svof_params_t *prm, const double *xf, const double *xc, 
   for (cudaEvent_t *e : s->branch_events())
     if (cudaSuccess != cudaEventCreateWithFlags(e, cudaEventDisableTiming)) return fail("event"), bail();
   // predict launch shape: rows per block.  A block's time is latency (its
-  // loads about 6 us, a cell a thread 2.2, a line a warp 3), so the rows are
-  // those with the least waves times that, over the blocks an SM holds by
-  // shared memory and registers (three of 256 threads).  us a substep of the
+  // loads about 6 us, a cell a thread 2.2, a line a warp 3, a line a thread 0.4
+  // and 0.063 a row), so the rows are those with the least waves times that,
+  // over the blocks an SM holds by shared memory and registers (three of 256
+  // threads), and the lines a thread's where that is the shorter: up to 41
+  // cells, and longer where a warp would have several.  us a substep of the
   // predictor and its tables, against ny / 148 rows: 256^2 28 -> 22, 512^2 49
-  // -> 38, 100 x 1024 34 -> 26, 1024 x 256 110 -> 57.
+  // -> 38, 100 x 1024 34 -> 26, 1024 x 256 110 -> 57.  A call of the predictor,
+  // a warp / a thread a line: 16 x 2048 33.4 / 28.8, 32 x 8192 65.4 / 43.5, 64 x
+  // 4096 61.2 / 45.8, 64 x 256 31.8 / 33.2, 128 x 256 33.4 / 38.5.
   {
     const long per_row = 6L * (nx + 1);
     const long fixed = 9L * (nx + 1);
@@ -644,12 +649,14 @@ int engine_create(const svof_params_t *prm, const double *xf, const double *xc, 
       const long threads = r * nx > 128 ? 256 : 128;
       const long held = 148 * std::max(1L, std::min(768 / threads, 227 / (kb(r) + 1)));
       const long blocks = (ny + r - 1) / r;
-      const long us = 60 + 22 * ((r * nx + threads - 1) / threads) + 30 * ((3 * r + threads / 32 - 1) / (threads / 32));
+      const long by_warps = 30 * ((3 * r + threads / 32 - 1) / (threads / 32)), by_threads = 4 + 63L * nx / 100;
+      const long us = 60 + 22 * ((r * nx + threads - 1) / threads) + std::min(by_warps, by_threads);
       const long cost = (blocks + held - 1) / held * us;
       if (best < 0 || cost < best) {
         best = cost;
         s->pred_rows = (int)r;
         s->pred_threads = (int)threads;
+        s->pred_thread_lines = by_threads < by_warps;
       }
     }
     s->pred_smem = predict_smem_bytes(nx, s->pred_rows);

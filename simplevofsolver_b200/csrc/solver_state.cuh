@@ -68,6 +68,7 @@ struct svof_solver {
   bool pred_lines = false;
   svof::DevBuf fw;
   int pred_rows = 1;
+  bool pred_thread_lines = false;
   int pred_threads = 256;
   size_t pred_smem = 0;
   // time step

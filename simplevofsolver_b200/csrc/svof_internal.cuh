@@ -97,7 +97,7 @@ struct PredictArgs {
   // vof the field after this substep's advection
   const double *vof;
   double grav_vof, vof_ref;
-  int rows_per_block;
+  int rows_per_block, thread_lines;  // thread_lines: a thread a line sweeps (else a warp)
   Grid2 g;
 };
 __global__ void k_predict(PredictArgs a);

@@ -191,6 +191,26 @@ __device__ __forceinline__ void line_solve(const T *__restrict__ L, const T *__r
   __syncwarp();
 }
 
+// The same for a line by the calling thread alone, in place
+template <class T>
+__device__ __forceinline__ void line_solve_thread(const T *__restrict__ L, const T *__restrict__ R,
+                                                  const T *__restrict__ V, int n, T *__restrict__ x) {
+  T v = x[0] / R[0];
+  x[0] = v;
+#pragma unroll 4
+  for (int i = 1; i < n - 1; i++) {
+    v = R[i] * (x[i] - L[i] * v);
+    x[i] = v;
+  }
+  const T r = R[n - 1];
+  x[n - 1] = v = (T(0.) != r) ? r * (x[n - 1] - L[n - 1] * v) : T(0.);
+#pragma unroll 4
+  for (int i = n - 2; i >= 0; i--) {
+    v = x[i] - V[i] * v;
+    x[i] = v;
+  }
+}
+
 // The same for 32 / LPL lines of a warp at once, LPL lanes a line, in place:
 // x[0 .. n-1] is the line of the calling lane (its group's), src its right-hand
 // side in global memory, read again only by lanes that have to repeat their
