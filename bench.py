@@ -696,8 +696,8 @@ def run3d(args, wl, ic, env, world, rank, local_rank):
             "config": {"workload": args.workload, "nx": n, "ny": n, "nz": n, "droplets": wl["ndrops"],
                        "radii": list(wl["radii"]), "x_grid": "tanh-stretched (1.5)",
                        "poisson": "r2c-y + dft-z + thomas-x, FP64 in both paths",
-                       "precision": "mixed (FP32 interface geometry, forces, sources and increments; FP64 state, "
-                                    "stencils, x line solves and Poisson solve)",
+                       "precision": "mixed (FP32 interface geometry, forces, sources, increments and their x sweeps; "
+                                    "FP64 state, stencils and Poisson solve)",
                        "l2": "not flushed: inputs larger than L2 (fields of %.1f GB resident)" % (
                            35.5 * cells * 8 / 1e9),
                        "parallelism": f"replicas{world}"},

@@ -95,7 +95,8 @@ template <class S>
 cudaError_t adj3_corners_launch(cudaStream_t st, const double *vof, const S *am, const S *akap, S *gbar,
                                 double *avof, AGrid3 ag);
 
-// deterministic sum (one block of 256 threads)
+// deterministic sum: shares of kAdjSumBlocks blocks of 256 threads, then one
+// block over the shares
 constexpr int kAdjSumBlocks = 592;
 __global__ void k3_adj_sum(const double *__restrict__ x, long n, double *__restrict__ out);
 // *dst = v in stream order

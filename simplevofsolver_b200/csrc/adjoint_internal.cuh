@@ -53,7 +53,8 @@ __global__ void k_adj_interface(AdjIfaceArgs a);
 constexpr int CBX = 32, CBY = 8;
 __global__ void k_adj_corners(const double *__restrict__ vof, const double *__restrict__ am,
                               const double *__restrict__ akap, double *__restrict__ avof, Grid2 g);
-// deterministic sum (one block of 256 threads)
+// deterministic sum: shares of kAdjSumBlocks blocks of 256 threads, then one
+// block over the shares
 constexpr int kAdjSumBlocks = 592;
 __global__ void k_adj_sum(const double *__restrict__ x, long n, double *__restrict__ out);
 // *dst = v in stream order

@@ -714,7 +714,11 @@ struct XlLong {
 struct XlShort {
   static constexpr int XLP = 8, MAXW = 24;
 };
-constexpr int kXlLongFrom = 321;  // cells a line
+// Cells a line from which 16 lanes have one.  us a step, 8 / 16 lanes, x 128 x
+// 128 FP64: 256 2153 / 2235, 320 2789 / 2817, 384 3335 / 3257, 512 4290 / 4094;
+// mixed: 256 1852 / 1918, 320 2395 / 2437, 384 2829 / 2845, 448 3322 / 3334, 512
+// 3656 / 3572; x 64 x 64 FP64: 256 730 / 739, 320 880 / 870, 384 1004 / 969.
+constexpr int kXlLongFrom = 321;
 // rows ahead of a segment
 template <class R>
 constexpr int kXlWarm = 4 == sizeof(R) ? 16 : 24;

@@ -582,7 +582,7 @@ __global__ void __launch_bounds__(CBX * CBY) k_adj_corners(const double *__restr
 
 // deterministic sum of n values: block b's share into out[b] (a thread's
 // values in order, the threads by a fixed tree); the callers sum kAdjSumBlocks
-// shares in a second launch (one block alone took 1.2 ms at 128^3)
+// shares in a second launch
 __global__ void k_adj_sum(const double *__restrict__ x, long n, double *__restrict__ out) {
   __shared__ double part[256];
   double s = 0.;

@@ -668,7 +668,10 @@ int engine_create(const svof_params_t *prm, const double *xf, const double *xc, 
     // large grids of long rows take the line-streaming predictor: the fused
     // kernel's blocks then hold an SM each for a row or two.  us a step, fused
     // against lines: 512^2 302 / 364, 300 x 2048 532 / 574, 512 x 2048 979 /
-    // 979, 1024 x 256 339 / 426, 1024 x 512 589 / 589, 1501 x 512 978 / 820,
+    // 979, 600 x 1024 552 / 625, 768 x 1024 722 / 731, 769 x 1024 747 / 742, 940 x
+    // 1024 856 / 857, 960 x 1024 1019 / 865 (an SM then holds one block in place
+    // of two), 700 x 2048 1141 / 1041, 769 x 2048 1249 / 1142, 1024 x 256 339 /
+    // 426, 1024 x 400 526 / 522, 1024 x 512 589 / 598, 1501 x 512 978 / 820,
     // 1024^2 1139 / 956.  SVOF_PREDICT_LINES = 0 / 1 forces either form (tests
     // compare them).
     s->pred_lines = (long)nx * ny >= 1L << 19 && nx > 768;
@@ -708,7 +711,7 @@ int engine_create(const svof_params_t *prm, const double *xf, const double *xc, 
     if (cudaSuccess != raise_smem_limit(k_dct_ysolve, sm)) return fail("cudaFuncSetAttribute(k_dct_ysolve)"), bail();
   }
   // launch plan checks: every dynamic shared-memory size covers what the
-  // kernel indexes, every line solve has a thread per line
+  // kernel indexes, the y line solve has a thread per line
   {
     const size_t need_pred = sizeof(double) * (6 * (size_t)s->pred_rows + 9) * (nx + 1);
     if (s->pred_smem < need_pred || s->pred_rows < 1)

@@ -429,9 +429,11 @@ int launch_project(svof3d_solver *s, int rk, int do_vel, int do_p) {
 // substep k (the advection waits for the previous projection, the predictor
 // for its force, and for the advected vof where that is buoyant, the next
 // force for the predictor that still reads this one's arrays).  Larger grids
-// fill the chip with each kernel and lose by it.  In line against two
-// branches: 61 x 64 x 32 four steps 1292 / 1076 us, 128^3 mixed restart stream
-// 9.12 / 8.81 ms, 256^3 step 8.40 / 8.47, 512^3 63.3 / 65.9 ms.  The three
+// fill the chip with each kernel, and the largest lose by it.  us a step in
+// line / on two branches: 64^3 FP64 360 / 308, 128^3 1321 / 1202, 256 x 128 x 128
+// 2335 / 2152, 256 x 256 x 128 4087 / 3975, 256^3 7718 / 7609, 512^3 (before
+// k3_xlines) 63300 / 65900; mixed 324 / 275, 1125 / 1036, 1990 / 1852, 3542 /
+// 3430, 6623 / 6545.  The three
 // substeps' predictor coefficients need dt alone and have a branch of their
 // own at every size (a launch of 8 us a substep at 256 rows).
 // tape (may be empty): called with (substep, stream, the interface's branch)
